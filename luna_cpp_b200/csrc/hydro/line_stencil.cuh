@@ -21,6 +21,7 @@ struct LineDev {
     double step;
     const double* __restrict__ gap;       // [n + 1]: gap[s + 1] from slot s to s + 1 in grid steps; gap[0], gap[n] over the ends
     const double* __restrict__ volume;    // [n]
+    const double* __restrict__ inv_volume;  // [n]: 1 / volume (the static line's step)
     const double* __restrict__ centroid;  // [n]: the centroid's offset from the generator
     luna::GasDev gas;
 };
