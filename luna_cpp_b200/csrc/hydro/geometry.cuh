@@ -51,10 +51,12 @@ struct alignas(32) FaceRow32 {
 template <class G>
 using FaceRow = typename std::conditional<sizeof(G) == sizeof(double), FaceRow64, FaceRow32>::type;
 
-// A staged row in shared memory (12 doubles, 96 B): the cell's primitive row (W, c, r, pad: as in HBM), then its
-// generator (D doubles).
-constexpr int kStagedDoubles = 12;
-constexpr int kStagedPos = 8;
+// A staged row in shared memory (10 doubles, 80 B): the cell's primitive row without its pad (W, c, r; in 2D one pad
+// double), then its generator (D doubles). 80 B are five 16-B units, an odd number: the rows that a warp's lanes read
+// at random start in all eight 16-B bank groups (96-B rows, six units, started in four of them: the sweep's L1 wavefronts
+// 49 -> 36 % of peak at 64^3, the 128^3 static step 1.80 -> 1.74 ms, with the compares below).
+constexpr int kStagedDoubles = 10;
+constexpr int kStagedPos = 7;
 
 template <int D, class G>
 struct GeometryDev {
@@ -448,7 +450,8 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                 double* dst = rows + R * (r0 + b * kTileCells + static_cast<int>(threadIdx.x));
                 const double* src = prims + PS * static_cast<int64_t>(cell[b]);
 #pragma unroll
-                for (int q = 0; q < PS; q += 2) cp_async16(dst + q, src + q);
+                for (int q = 0; q < 6; q += 2) cp_async16(dst + q, src + q);
+                if constexpr (D == 3) cp_async8(dst + 6, src + 6);
 #pragma unroll
                 for (int a = 0; a < D; ++a) cp_async8(dst + kStagedPos + a, m.pos + D * static_cast<int64_t>(cell[b]) + a);
             }
@@ -515,7 +518,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                 const bool owned = (word[b] & kOwnedBit) != 0, tiny_face = (word[b] & kTinyBit) != 0;
                 any_tiny = any_tiny || tiny_face;
                 const double* rj = rows + R * static_cast<int>(word[b] & kIndexMask);
-                double pj[8];
+                double pj[kStagedDoubles];
 #pragma unroll
                 for (int q = 0; q < 6; q += 2) {
                     const double2 w2 = *reinterpret_cast<const double2*>(rj + q);
@@ -523,14 +526,17 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                     pj[q + 1] = w2.y;
                 }
                 if (owned) {  // FaceStep (finite_volume.hpp:1074-1090)
-                    const double2 w2 = *reinterpret_cast<const double2*>(rj + 6);
-                    pj[6] = w2.x;
-                    pj[7] = w2.y;
+#pragma unroll
+                    for (int q = 6; q < kStagedDoubles; q += 2) {  // the radius (3D) and the generator
+                        const double2 w2 = *reinterpret_cast<const double2*>(rj + q);
+                        pj[q] = w2.x;
+                        pj[q + 1] = w2.y;
+                    }
                     double dv[D], d[D];
 #pragma unroll
                     for (int a = 0; a < D; ++a) {
                         dv[a] = pj[1 + a] - Wi[1 + a];
-                        d[a] = m.wrap(rj[kStagedPos + a] - own_at(kStagedPos + a), a);  // Geometry::separation of owner and neighbour
+                        d[a] = m.wrap(pj[kStagedPos + a] - own_at(kStagedPos + a), a);  // Geometry::separation of owner and neighbour
                     }
                     const double dist = sqrt(dot<D>(d, d));
                     // Both cells' terms: the smaller radius gives the smaller one. den > 0 is vsig > 0.
@@ -549,8 +555,9 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                         for (int a = 0; a < D; ++a) g[D * v + a] += c[b][a] * dWg;
                         if (!tiny_face) {
                             const G value = exact ? static_cast<G>(pj[v]) : dWg;
-                            lo[v] = fmin(lo[v], value);
-                            hi[v] = fmax(hi[v], value);
+                            // compares and selects: fmin and fmax spend more on NaN (which neither form takes in)
+                            lo[v] = value < lo[v] ? value : lo[v];
+                            hi[v] = value > hi[v] ? value : hi[v];
                         }
                     }
                 }

@@ -15,8 +15,12 @@
 namespace luna {
 
 constexpr int kTileCells = 128;  // cells (threads) of a tile: one block
-constexpr int kTileRows = 416;   // staged rows a tile may use (39 KB of shared memory); a cell alone needing more gets a
+constexpr int kTileRows = 416;   // staged rows a tile may use (33 KB of shared memory); a cell alone needing more gets a
                                  // tile of its own, swept by a second launch with more shared memory
+constexpr int kDeviceTileRows = 640;  // the same of the device cut, which takes its cells as they come and so stages
+                                      // more: 51 KB, the most that leaves four blocks an SM
+                                      // (61 x 47 x 53 cells: with 416 a tenth of the tiles were a second launch behind
+                                      // the first, its 4 steps 914 us; now 839)
 constexpr int kBigTileRows = 2360;  // the most rows one block can stage (227 KB); a mesh with a larger list is refused
 
 struct SweepTiles {
@@ -73,7 +77,7 @@ std::string build_tile_faces(int64_t n_cells, int64_t n_faces, int64_t tiles, co
 
 // The same tiles cut on the device from a device mesh, for a mesh that is rebuilt every step (the moving mesh's
 // remesh): the cells of a tile are 128 consecutive cells of the Morton order (no greedy cut), within a tile by list
-// length, longest first; a tile staging more than kTileRows rows goes with the single-cell tiles of the host cut to the
+// length, longest first; a tile staging more than kDeviceTileRows rows goes with the single-cell tiles of the host cut to the
 // second launch. The sweep's results do not depend on the tiling (the staged rows are copies of HBM rows).
 struct DeviceTilePlan {
     int64_t tiles = 0, normal_tiles = 0, staged = 0, slots = 0;

@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
             if (rows > luna::kBigTileRows)
                 atomicOr(&plan.ctr->overflow, 1);
             else
-                atomicMax(rows > luna::kTileRows ? &plan.ctr->big_rows : &plan.ctr->normal_rows, rows);
+                atomicMax(rows > luna::kDeviceTileRows ? &plan.ctr->big_rows : &plan.ctr->normal_rows, rows);
         }
     } else {
         // the halo by cell index (bitonic, ascending)
@@ -262,7 +262,7 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
 __global__ void k_tile_flags(int64_t T, const int32_t* __restrict__ rows, int32_t* __restrict__ normal, int32_t* __restrict__ big) {
     const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (t > T) return;
-    const bool is_big = t < T && rows[t] > luna::kTileRows;
+    const bool is_big = t < T && rows[t] > luna::kDeviceTileRows;
     normal[t] = t < T && !is_big;
     big[t] = is_big;
 }
@@ -279,7 +279,7 @@ __global__ void k_tile_place(int64_t T, const int32_t* __restrict__ rows, const 
         return;
     }
     const int32_t normals = normal_before[T];
-    const bool is_big = rows[t] > luna::kTileRows;
+    const bool is_big = rows[t] > luna::kDeviceTileRows;
     const int32_t u = is_big ? normals + big_before[t] : normal_before[t];
     pos[t] = u;
     rows_u[u] = rows[t];
