@@ -200,7 +200,8 @@ LUNA_API luna_status luna_fv_limiter_inputs(luna_fv* fv, void* features, double*
  * cores (tcgen05, accumulators in tensor memory); it synchronises the stream to read its completion status
  * (LUNA_ETIMEOUT if a bounded wait gave up). train_step: the gradient of scale * sum w (sigmoid(o) - t)^2 over rows
  * (targets t and weights w FP32 [n][5]) into grad, the loss into *loss (device); workspace of
- * luna_mlp_train_workspace_floats(n) floats; deterministic. adam: one Adam update (step counts from 1). */
+ * luna_mlp_train_workspace_floats(n) floats; deterministic. train_step_mean: the same with scale = 1 / max(sum w, 1e-30),
+ * summed on the device (no read of the weights by the host). adam: one Adam update (step counts from 1). */
 LUNA_API int64_t luna_mlp_param_count(void);
 /* The polls a tensor-core completion wait of the learned limiter's forward makes before it gives up (LUNA_ETIMEOUT from
  * luna_mlp_forward and from the learned step's luna_fv_time_step), for every later launch in this process; < 0 restores
@@ -211,6 +212,8 @@ LUNA_API int64_t luna_mlp_train_workspace_floats(int64_t n);
 LUNA_API luna_status luna_mlp_forward(const float* params, const void* features, int64_t n, float* logits, void* stream);
 LUNA_API luna_status luna_mlp_train_step(const float* params, const void* features, const float* target, const float* weight, int64_t n,
                                          float scale, float* grad, float* loss, float* workspace, int64_t workspace_floats, void* stream);
+LUNA_API luna_status luna_mlp_train_step_mean(const float* params, const void* features, const float* target, const float* weight, int64_t n,
+                                              float* grad, float* loss, float* workspace, int64_t workspace_floats, void* stream);
 LUNA_API luna_status luna_mlp_adam(float* params, const float* grad, float* m, float* v, float lr, float beta1, float beta2, float eps,
                                    int step, void* stream);
 

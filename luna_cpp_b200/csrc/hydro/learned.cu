@@ -70,7 +70,7 @@ LUNA_API int luna_mlp_set_wait_limit(int polls) {
 
 LUNA_API int64_t luna_mlp_train_workspace_floats(int64_t n) {
     const int64_t blocks = (n + luna::mlp::kRowsPerBlock - 1) / luna::mlp::kRowsPerBlock;
-    return blocks * (luna::mlp::kParams + 1);
+    return blocks * (luna::mlp::kParams + 2);  // a gradient, a loss and a sum of weights a block
 }
 
 LUNA_API luna_status luna_mlp_forward(const float* params, const void* features, int64_t n, float* logits, void* stream) {
@@ -92,28 +92,39 @@ LUNA_API luna_status luna_mlp_forward(const float* params, const void* features,
     return LUNA_OK;
 }
 
+static luna_status train_step(const char* what, const float* params, const void* features, const float* target, const float* weight, int64_t n,
+                              bool mean, float scale, float* grad, float* loss, float* workspace, int64_t workspace_floats, void* stream) {
+    using namespace luna::mlp;
+    if (!params || !features || !target || !weight || !grad || !loss || !workspace || n <= 0 || n >= (int64_t(1) << 31))
+        return fail(LUNA_EINVAL, std::string(what) + ": bad argument");
+    const int64_t turns = (n + kRowsPerBlock - 1) / kRowsPerBlock;
+    if (workspace_floats < turns * (kParams + (mean ? 2 : 1))) return fail(LUNA_EINVAL, std::string(what) + ": workspace too small");
+    cudaStream_t s = static_cast<cudaStream_t>(stream);
+    const int smem = static_cast<int>(sizeof(SmemTrain));
+    const cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+    if (e != cudaSuccess) return fail(LUNA_ECUDA, std::string("k_mlp_train shared memory: ") + cudaGetErrorString(e));
+    // one wave of the blocks that share an SM, each taking further rows in turn: the slots stay few
+    const int blocks = static_cast<int>(turns < 148 * kTrainBlocksPerSm ? turns : 148 * kTrainBlocksPerSm);
+    float* slots = workspace;
+    float* loss_slots = workspace + static_cast<int64_t>(blocks) * kParams;
+    float* weight_slots = mean ? loss_slots + blocks : nullptr;
+    k_mlp_train<<<blocks, 128, smem, s>>>(params, static_cast<const __nv_bfloat16*>(features), target, weight, static_cast<int>(n), slots, loss_slots,
+                                          weight_slots);
+    const luna_status st = check_launch("k_mlp_train");
+    if (st != LUNA_OK) return st;
+    k_mlp_reduce<<<(kParams + kReduceParams - 1) / kReduceParams, kReduceParams * kReduceGroups, 0, s>>>(slots, loss_slots, weight_slots, blocks,
+                                                                                                          scale, grad, loss);
+    return check_launch("k_mlp_reduce");
+}
+
 LUNA_API luna_status luna_mlp_train_step(const float* params, const void* features, const float* target, const float* weight, int64_t n,
                                          float scale, float* grad, float* loss, float* workspace, int64_t workspace_floats, void* stream) {
-    if (!params || !features || !target || !weight || !grad || !loss || !workspace || n <= 0 || n >= (int64_t(1) << 31))
-        return fail(LUNA_EINVAL, "luna_mlp_train_step: bad argument");
-    const int64_t blocks = (n + luna::mlp::kRowsPerBlock - 1) / luna::mlp::kRowsPerBlock;
-    if (workspace_floats < blocks * (luna::mlp::kParams + 1)) return fail(LUNA_EINVAL, "luna_mlp_train_step: workspace too small");
-    cudaStream_t s = static_cast<cudaStream_t>(stream);
-    const int smem = static_cast<int>(sizeof(luna::mlp::SmemTrain));
-    static bool configured = false;
-    if (!configured) {
-        const cudaError_t e = cudaFuncSetAttribute(luna::mlp::k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-        if (e != cudaSuccess) return fail(LUNA_ECUDA, std::string("k_mlp_train shared memory: ") + cudaGetErrorString(e));
-        configured = true;
-    }
-    float* slots = workspace;
-    float* loss_slots = workspace + blocks * luna::mlp::kParams;
-    luna::mlp::k_mlp_train<<<static_cast<int>(blocks), 128, smem, s>>>(params, static_cast<const __nv_bfloat16*>(features), target, weight,
-                                                                      static_cast<int>(n), slots, loss_slots);
-    luna_status st = check_launch("k_mlp_train");
-    if (st != LUNA_OK) return st;
-    luna::mlp::k_mlp_reduce<<<(luna::mlp::kParams + 255) / 256, 256, 0, s>>>(slots, loss_slots, static_cast<int>(blocks), scale, grad, loss);
-    return check_launch("k_mlp_reduce");
+    return train_step("luna_mlp_train_step", params, features, target, weight, n, false, scale, grad, loss, workspace, workspace_floats, stream);
+}
+
+LUNA_API luna_status luna_mlp_train_step_mean(const float* params, const void* features, const float* target, const float* weight, int64_t n,
+                                              float* grad, float* loss, float* workspace, int64_t workspace_floats, void* stream) {
+    return train_step("luna_mlp_train_step_mean", params, features, target, weight, n, true, 1.0f, grad, loss, workspace, workspace_floats, stream);
 }
 
 LUNA_API luna_status luna_mlp_adam(float* params, const float* grad, float* m, float* v, float lr, float beta1, float beta2, float eps,

@@ -96,6 +96,7 @@ SIGNATURES = {
     "luna_mlp_train_workspace_floats": ([I64], I64),
     "luna_mlp_forward": ([P, P, I64, P, P], I),
     "luna_mlp_train_step": ([P, P, P, P, I64, ctypes.c_float, P, P, P, I64, P], I),
+    "luna_mlp_train_step_mean": ([P, P, P, P, I64, P, P, P, I64, P], I),
     "luna_mlp_adam": ([P, P, P, P, ctypes.c_float, ctypes.c_float, ctypes.c_float, ctypes.c_float, I, P], I),
     "luna_fv_timings": ([P, P, I], I),
     "luna_mesh_tiles": ([P, P, P, P, P, P, P], I),

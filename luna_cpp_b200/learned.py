@@ -55,13 +55,15 @@ class LimiterMLP:
     def gradient(self, features_bf16, target, weight, scale=None) -> float:
         """The gradient of sum w (sigmoid(o) - t)^2 * scale into self.grad (scale default 1 / sum w); returns the loss."""
         n = features_bf16.shape[0]
-        if scale is None:
-            scale = 1.0 / max(float(weight.sum().item()), 1e-30)
         need = int(lib().luna_mlp_train_workspace_floats(n))
         if self._workspace is None or self._workspace.numel() < need:
             self._workspace = torch.empty(need, dtype=torch.float32, device=features_bf16.device)
-        hydro.check(lib().luna_mlp_train_step(_ptr(self.params), _ptr(features_bf16), _ptr(target), _ptr(weight), n, scale,
-                                              _ptr(self.grad), _ptr(self.loss), _ptr(self._workspace), need, _stream()))
+        data = (_ptr(self.params), _ptr(features_bf16), _ptr(target), _ptr(weight), n)
+        out = (_ptr(self.grad), _ptr(self.loss), _ptr(self._workspace), need, _stream())
+        if scale is None:
+            hydro.check(lib().luna_mlp_train_step_mean(*data, *out))
+        else:
+            hydro.check(lib().luna_mlp_train_step(*data, scale, *out))
         return self.loss
 
     def adam(self, lr=1e-3, beta1=0.9, beta2=0.999, eps=1e-8):

@@ -195,3 +195,31 @@ def test_tensor_core_wait_that_runs_out_reports_a_timeout(cuda):
     assert b"gave up" in lib.luna_last_error()
     want, _ = M.forward(p, x)
     assert rel(net.forward(feats).cpu().numpy(), want) < 2e-3
+
+
+@pytest.mark.parametrize("n", [1, 15, 64, 65, 18944, 19009, 40001])
+def test_gradient_over_blocks_and_turns(cuda, n):
+    """Row counts around a warp's 16, a block's 64 and one wave of blocks (296 of 64 rows: beyond it a block takes rows
+    in turns): loss and gradient against the oracle (BF16 operands, FP32 sums), the same bits twice, and the weights
+    summed on the device against the caller's scale."""
+    import torch
+
+    from luna_cpp_b200.learned import LimiterMLP, init_params
+
+    x, t, w = data(n, seed=n)
+    w[0] = 1.0
+    p = init_params(4)
+    net = LimiterMLP(p)
+    xd, td, wd = (torch.tensor(x, device="cuda").to(torch.bfloat16), torch.tensor(t, device="cuda"), torch.tensor(w, device="cuda"))
+    scale = 1.0 / float(w.sum())
+    want_loss, want_g = M.loss_and_grad(p, x, t, w, scale)
+    loss = net.gradient(xd, td, wd, scale).item()
+    g = net.grad.cpu().numpy().copy()
+    assert abs(loss - want_loss) <= 2e-3 * abs(want_loss)
+    assert rel(g, want_g) < 2e-3
+    mean_loss = net.gradient(xd, td, wd).item()
+    mean_g = net.grad.cpu().numpy().copy()
+    # one rounding of the sum of the weights (FP32, exact below 2^24 ones) and of its reciprocal
+    assert abs(mean_loss - loss) <= 1e-6 * abs(loss) and rel(mean_g, g) < 1e-6
+    net.gradient(xd, td, wd)
+    assert np.array_equal(net.grad.cpu().numpy(), mean_g)
