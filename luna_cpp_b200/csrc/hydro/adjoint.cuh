@@ -1,23 +1,100 @@
 // The adjoint of one static step (luna-cpp's step_adjoint, src/hydro/finite_volume.hpp:2201-2231): Qbar^n = J^T Qbar^n+1
-// at fixed dt, for the FP64 policy, order 1, the per-face loop. Four passes, no atomics (the same bits every run):
-//   k_sweep_fit      the forward sweep again, keeping the fit the gradient's adjoint needs (SweepFitHook<false>,
-//                    finite_volume.hpp:1763-1926): M's Cholesky factor, M's row 0, the unlimited gradient g0, per
-//                    variable the last clip (offset, bound, flags) and the face its bound came through;
+// at fixed dt, for the FP64 policy, order 1, the per-face loop. Four passes, no atomics (the same bits every run), over
+// the rows that the step itself streams (geometry.cuh: the gradient operator's c_k and the face offsets by tile, the face
+// rows, the merged W/g rows):
+//   k_sweep_fit      the forward sweep again, keeping what the gradient's adjoint needs (SweepFitHook<false>,
+//                    finite_volume.hpp:1763-1926): the unlimited gradient g0 and, per variable, the last clip (its entry
+//                    and flags), the bound and the entry that the bound came through;
 //   k_faces_adjoint  once per face: the Riemann adjoint -> the bars of both face states (AdjointFaces, :2078-2102);
-//   k_cell_adjoint   per cell, one walk: face-state adjoints -> W and g bars, the limited gradient's adjoint from the
-//                    stored fit -> the fit's b bars, bound bars, the cell's own W bar (AdjointCell, :2107-2169);
-//   k_gather_adjoint per cell: the neighbours' b and bound bars, then the primitive adjoint into Qbar (:2171-2195).
+//   k_cell_adjoint   per cell: face-state adjoints -> W and g bars, the limited gradient's adjoint (AdjointCell,
+//                    :2107-2169) -> g0's bar; g0 = sum_k c_k (W_k - W_i) then gives each neighbour c_k . g0bar and the
+//                    cell minus their sum: each neighbour's share (with the bound's bar at its entry) takes the place of
+//                    the cell's face-state bar in the face's row, which no other cell reads;
+//   k_gather_adjoint per cell: its neighbours' shares from its faces' rows, then the primitive adjoint into Qbar
+//                    (:2171-2195).
+// What the passes spend is gather instructions (an L1 line a lane and load), so every row is read in its widest loads and
+// none is read twice. Measured against the passes over the mesh arrays, which solved every fit by Cholesky and gathered
+// 20 bars and the geometry for each neighbour: at 72 x 64 x 60 cells one step_adjoint and one step_tangent 2.98 -> 1.96 ms
+// (k_sweep_fit 406 -> 195 us, k_gather_adjoint 261 -> 76, k_tangent_fluxes 467 -> 200, k_tangent_sweep 135 -> 84); 8 steps
+// of the 512^2 rollout with its backward 5.4 -> 4.2 ms.
 #pragma once
 
+#include "geometry.cuh"
 #include "kernels.cuh"
 
 namespace luna {
 
+// A cell's fit row: the unlimited gradient (V D doubles), then each variable's bound (V).
 template <int D>
 struct FitLayout {
-    static constexpr int U = D + 1, V = D + 2;
-    static constexpr int factor = 0, row0 = U * U, g0 = row0 + U, offset = g0 + V * D, bound = offset + V * D, width = bound + V;
+    static constexpr int V = D + 2;
+    static constexpr int g0 = 0, bound = V * D, width = bound + V;
 };
+// A variable's clip word: bit 0 clipped, 1 at the upper bound, 2 to zero; the last clip's entry; the entry of the bound
+// (a list has at most kBigTileRows entries).
+constexpr int kClipEntryBits = 14, kClipEntryMask = (1 << kClipEntryBits) - 1;
+static_assert(kBigTileRows <= kClipEntryMask, "a list entry fits its field of the clip word");
+__host__ __device__ constexpr int clip_word(int flags, int entry, int bound) { return flags | entry << 3 | bound << (3 + kClipEntryBits); }
+__host__ __device__ constexpr int clip_entry(int word) { return (word >> 3) & kClipEntryMask; }
+__host__ __device__ constexpr int bound_entry(int word) { return (word >> (3 + kClipEntryBits)) & kClipEntryMask; }
+// Doubles of one side of a face's bar row, and of a tangent's dW row: whole 16-B units.
+template <int D>
+constexpr int bar_stride() {
+    return D == 3 ? 6 : 4;
+}
+// Doubles a staged row of the derivative sweeps takes: V, padded to an odd number of 16-B units (see kStagedDoubles).
+constexpr int kFitStaged = 6;
+
+// V doubles of a row of bar_stride at p (16-B aligned) in 16-B loads and stores.
+template <int V>
+__device__ __forceinline__ void load_bar(const double* p, double* out) {
+#pragma unroll
+    for (int v = 0; v + 1 < V; v += 2) {
+        const double2 w = *reinterpret_cast<const double2*>(p + v);
+        out[v] = w.x;
+        out[v + 1] = w.y;
+    }
+    if constexpr (V % 2) out[V - 1] = p[V - 1];
+}
+template <int V>
+__device__ __forceinline__ void store_bar(double* p, const double* in) {
+#pragma unroll
+    for (int v = 0; v + 1 < V; v += 2) *reinterpret_cast<double2*>(p + v) = make_double2(in[v], in[v + 1]);
+    if constexpr (V % 2) p[V - 1] = in[V - 1];
+}
+// A merged row (W then g, wg_stride doubles, 32-B aligned) and its store.
+template <int D>
+__device__ __forceinline__ void load_wg(const double* rows, int i, double* W, double* g) {
+    constexpr int V = D + 2, S = wg_stride<D>();
+    double row[S];
+    const double* p = rows + static_cast<int64_t>(S) * i;
+#pragma unroll
+    for (int c = 0; c < S; c += 4) ldg256(p + c, row + c);
+#pragma unroll
+    for (int v = 0; v < V; ++v) W[v] = row[v];
+#pragma unroll
+    for (int c = 0; c < V * D; ++c) g[c] = row[V + c];
+}
+template <int D>
+__device__ __forceinline__ void store_wg(double* rows, int i, const double* W, const double* g) {
+    constexpr int V = D + 2, S = wg_stride<D>();
+    double2* p = reinterpret_cast<double2*>(rows + static_cast<int64_t>(S) * i);
+    const auto at = [&](int c) { return c < V ? W[c] : c < V + V * D ? g[c - V] : 0.0; };
+#pragma unroll
+    for (int c = 0; c < S; c += 2) p[c / 2] = make_double2(at(c), at(c + 1));
+}
+// The block's tile staged: kFitStaged doubles of each staged cell from its row of `stride` doubles (16-B aligned).
+template <int D>
+__device__ __forceinline__ void stage_rows(const GeometryDev<D, double>& geo, int tile, const double* __restrict__ from, int stride, double* rows) {
+    const int s0 = geo.stage_start[tile], staged = geo.stage_start[tile + 1] - s0;
+    for (int r = threadIdx.x; r < staged; r += kTileCells) {
+        const double* src = from + static_cast<int64_t>(stride) * geo.stage_cells[s0 + r];
+#pragma unroll
+        for (int q = 0; q < (D == 3 ? 6 : 4); q += 2) cp_async16(rows + kFitStaged * r + q, src + q);
+    }
+    cp_async_wait_all();
+    __syncthreads();
+}
 
 // primitive_adjoint (euler.hpp:143-162).
 template <int D>
@@ -353,139 +430,84 @@ __device__ __forceinline__ bool side_value(const double* W, const double* g, con
     return fallback;
 }
 
-// Resident blocks an SM the adjoint's register-heavy kernels are cut for, and the list entries the gather requests
-// together. Measured at 128^3 (step_adjoint, FP64): no cap (128-164 registers) 9.66 ms, 4 blocks (128 registers, a few
-// spills) 8.32 ms; a gather batch of 4 changed nothing (9.68 / 8.34 ms); 3 blocks 8.65 ms, and the fit's entry loop
-// unrolled by 2 8.54 ms (8.28 for the default).
 #ifndef LUNA_ADJ_MIN_BLOCKS
-#define LUNA_ADJ_MIN_BLOCKS 4
-#endif
-#ifndef LUNA_ADJ_GATHER_BATCH
-#define LUNA_ADJ_GATHER_BATCH 1
+#define LUNA_ADJ_MIN_BLOCKS 4  // resident blocks an SM the adjoint's register-heavy kernels are cut for
 #endif
 
-// The sweep again with the fit kept (Sweep<false, true, SweepFitHook<false>>): the same gradients as k_sweep's FP64
-// policy, plus fit rows [N][FitLayout::width] and flags [N][2V] (clipped | upper << 1 | zero << 2; the bound's face).
+// The sweep again with the fit kept (Sweep<false, true, SweepFitHook<false>>), one block a tile as k_sweep_tiles: the
+// merged rows W, g (limited in list order: no round-off rule, so that every clip is the reference's), the fit rows
+// [N][FitLayout::width] and the clip words [N][V].
 template <int D, bool Limit>
-__global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(MeshDev<D> m, const double* __restrict__ prims, double* __restrict__ grad_out,
-                                                   double* __restrict__ fit, int32_t* __restrict__ flags) {
-    constexpr int V = D + 2, U = D + 1, GS = grad_stride<D>();
+__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
+                                                                             const double* __restrict__ prims, double* __restrict__ wg,
+                                                                             double* __restrict__ fit, int32_t* __restrict__ clip) {
+    constexpr int V = D + 2;
     using FL = FitLayout<D>;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.n) return;
-    const double* pi = prims + PS * i;
-    double Wi[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) Wi[v] = pi[v];
-    double surface = 0, smallest = __longlong_as_double(0x7ff0000000000000ll);
-    double lo[V], hi[V];
-    int lo_f[V], hi_f[V];
-    double M[U][U], b[V][U];
+    extern __shared__ double2 staged_rows[];
+    double* rows = reinterpret_cast<double*>(staged_rows);
+    const int tile = tile0 + static_cast<int>(blockIdx.x);
+    stage_rows<D>(geo, tile, prims, PS, rows);
+    const int64_t t = static_cast<int64_t>(tile) * kTileCells + threadIdx.x;
+    const int i = geo.order[t];
+    if (i < 0) return;
+    const int count = m.start[i + 1] - m.start[i];
+    const int64_t slot0 = static_cast<int64_t>(geo.slice_base[t >> 5]) * 32 + (t & 31);
+    const unsigned long long once = l2_evict_first();
+    double Wi[V], lo[V], hi[V], g[V * D];
+    int lo_k[V], hi_k[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
+        Wi[v] = rows[kFitStaged * threadIdx.x + v];
         lo[v] = finite_max<double>();
         hi[v] = -finite_max<double>();
-        lo_f[v] = hi_f[v] = -1;
+        lo_k[v] = hi_k[v] = 0;
 #pragma unroll
-        for (int p = 0; p < U; ++p) b[v][p] = 0;
+        for (int a = 0; a < D; ++a) g[D * v + a] = 0;
     }
+    bool any_tiny = false;
+    for (int k = 0; k < count; ++k) {
+        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
+        const unsigned int word = geo.nbr[slot];
+        const double2 c01 = geo.c01[slot];
+        double c[D];
+        c[0] = c01.x;
+        c[1] = c01.y;
+        if constexpr (D == 3) c[2] = geo.c2[slot];
+        const double* rj = rows + kFitStaged * static_cast<int>(word & kIndexMask);
+        double Wj[kFitStaged];
 #pragma unroll
-    for (int p = 0; p < U; ++p)
-#pragma unroll
-        for (int s = 0; s < U; ++s) M[p][s] = 0;
-    double centroid[D];
-#pragma unroll
-    for (int a = 0; a < D; ++a) centroid[a] = m.cen[D * i + a];
-    const int first = m.start[i], end = m.start[i + 1];
-    for (int k = first; k < end; ++k) {
-        const int32_t e = m.list[k];
-        const int f = list_face(e);
-        const int j = e >= 0 ? m.neighbour[f] : m.owner[f];
-        const double* pj = prims + PS * j;
-        double d[D];
-        m.separation(i, j, d);
-        const double magnitude = m.mag[f];
-        surface += magnitude;
-        smallest = fmin(smallest, magnitude);
-        double X[U];
-        X[0] = 1;
-#pragma unroll
-        for (int p = 1; p < U; ++p) X[p] = d[p - 1] + m.cen[D * j + p - 1] - centroid[p - 1];
-#pragma unroll
-        for (int p = 0; p < U; ++p)
-#pragma unroll
-            for (int s = p; s < U; ++s) M[p][s] += magnitude * X[p] * X[s];
+        for (int q = 0; q < (D == 3 ? 6 : 4); q += 2) {
+            const double2 w2 = *reinterpret_cast<const double2*>(rj + q);
+            Wj[q] = w2.x;
+            Wj[q + 1] = w2.y;
+        }
+        const bool tiny_face = (word & kTinyBit) != 0;
+        any_tiny = any_tiny || tiny_face;
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            const double Wj = pj[v];
-            const double dW = Wj - Wi[v];
+            const double dW = Wj[v] - Wi[v];
 #pragma unroll
-            for (int p = 0; p < U; ++p) b[v][p] += magnitude * X[p] * dW;
-            if (Wj < lo[v]) lo[v] = Wj, lo_f[v] = f;
-            if (Wj > hi[v]) hi[v] = Wj, hi_f[v] = f;
-        }
-    }
-    const double tiny = 1e-6 * surface;
-    const bool any_tiny = smallest < tiny;
-    if (any_tiny) {
-#pragma unroll
-        for (int v = 0; v < V; ++v) {
-            lo[v] = finite_max<double>();
-            hi[v] = -finite_max<double>();
-        }
-        for (int k = first; k < end; ++k) {
-            const int32_t e = m.list[k];
-            const int f = list_face(e);
-            if (m.mag[f] < tiny) continue;
-            const int j = e >= 0 ? m.neighbour[f] : m.owner[f];
-            const double* pj = prims + PS * j;
-#pragma unroll
-            for (int v = 0; v < V; ++v) {
-                if (pj[v] < lo[v]) lo[v] = pj[v], lo_f[v] = f;
-                if (pj[v] > hi[v]) hi[v] = pj[v], hi_f[v] = f;
+            for (int a = 0; a < D; ++a) g[D * v + a] += c[a] * dW;
+            if (!tiny_face) {  // neighbour_range (finite_volume.hpp:572-588) leaves the tiny faces out
+                if (Wj[v] < lo[v]) lo[v] = Wj[v], lo_k[v] = k;
+                if (Wj[v] > hi[v]) hi[v] = Wj[v], hi_k[v] = k;
             }
         }
     }
     double* fr = fit + static_cast<int64_t>(FL::width) * i;
-    {  // cholesky (finite_volume.hpp:677-687), kept in the fit row
-        double Lc[U][U];
+    store_bar<V * D>(fr + FL::g0, g);
+    int flag[V], clip_k[V];
 #pragma unroll
-        for (int p = 0; p < U; ++p)
-#pragma unroll
-            for (int s = 0; s < U; ++s) Lc[p][s] = 0;
-#pragma unroll
-        for (int p = 0; p < U; ++p)
-#pragma unroll
-            for (int s = 0; s <= p; ++s) {
-                double sum = M[s][p];
-#pragma unroll
-                for (int k = 0; k < s; ++k) sum -= Lc[p][k] * Lc[s][k];
-                Lc[p][s] = p == s ? sqrt(sum) : sum / Lc[s][s];
-            }
-#pragma unroll
-        for (int p = 0; p < U; ++p) {
-#pragma unroll
-            for (int s = 0; s < U; ++s) fr[FL::factor + p * U + s] = Lc[p][s];
-            fr[FL::row0 + p] = M[0][p];
-        }
-    }
-    double g[V * D];
-    cholesky_solve<D, double>(M, b, g);
-#pragma unroll
-    for (int c = 0; c < V * D; ++c) fr[FL::g0 + c] = g[c];
-    bool clipped[V], upper[V], zero[V];
-    int clip_f[V];
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        clipped[v] = upper[v] = zero[v] = false;
-        clip_f[v] = -1;
-    }
+    for (int v = 0; v < V; ++v) flag[v] = clip_k[v] = 0;
     if constexpr (Limit) {
-        for (int k = first; k < end; ++k) {
-            const int f = list_face(m.list[k]);
-            if (any_tiny && m.mag[f] < tiny) continue;
+        for (int k = 0; k < count; ++k) {
+            const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
+            if (any_tiny && (geo.nbr[slot] & kTinyBit)) continue;
+            const double2 o01 = ldg_hint(geo.off01 + slot, once);
             double offset[D];
-            m.face_offset(f, i, offset);
+            offset[0] = o01.x;
+            offset[1] = o01.y;
+            if constexpr (D == 3) offset[2] = ldg_hint(geo.off2 + slot, once);
 #pragma unroll
             for (int v = 0; v < V; ++v) {
                 double* gv = g + D * v;
@@ -494,235 +516,198 @@ __global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(MeshDev<
                     const double s = hi[v] > Wi[v] ? (hi[v] - Wi[v]) / dp : 0.0;
 #pragma unroll
                     for (int a = 0; a < D; ++a) gv[a] = gv[a] * s;
-                    clipped[v] = true, upper[v] = true, zero[v] = !(hi[v] > Wi[v]), clip_f[v] = f;
+                    flag[v] = hi[v] > Wi[v] ? 3 : 7, clip_k[v] = k;
                 } else if (dp < 0 && Wi[v] + dp < lo[v]) {
                     const double s = lo[v] < Wi[v] ? (lo[v] - Wi[v]) / dp : 0.0;
 #pragma unroll
                     for (int a = 0; a < D; ++a) gv[a] = gv[a] * s;
-                    clipped[v] = true, upper[v] = false, zero[v] = !(lo[v] < Wi[v]), clip_f[v] = f;
+                    flag[v] = lo[v] < Wi[v] ? 1 : 5, clip_k[v] = k;
                 }
             }
         }
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-        double offset[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) offset[a] = 0;
-        if (clipped[v]) m.face_offset(clip_f[v], i, offset);
-#pragma unroll
-        for (int a = 0; a < D; ++a) fr[FL::offset + D * v + a] = offset[a];
-        fr[FL::bound + v] = upper[v] ? hi[v] : lo[v];
-        flags[2 * V * i + v] = (clipped[v] ? 1 : 0) | (upper[v] ? 2 : 0) | (zero[v] ? 4 : 0);
-        flags[2 * V * i + V + v] = upper[v] ? hi_f[v] : lo_f[v];
+        const bool upper = (flag[v] & 2) != 0;
+        fr[FL::bound + v] = upper ? hi[v] : lo[v];
+        clip[V * static_cast<int64_t>(i) + v] = clip_word(flag[v], clip_k[v], upper ? hi_k[v] : lo_k[v]);
     }
-    double* out = grad_out + static_cast<int64_t>(GS) * i;
-#pragma unroll
-    for (int c = 0; c < V * D; ++c) out[c] = g[c];
+    store_wg<D>(wg, i, Wi, g);
 }
 
-// AdjointFaces (finite_volume.hpp:2078-2102): per face, the bars of its two face states from Qbar's jump across it.
+// AdjointFaces (finite_volume.hpp:2078-2102): per face, the bars of its two face states from Qbar's jump across it, into
+// the face's row of two sides.
 template <int D, int Riemann>
-__global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_faces_adjoint(MeshDev<D> m, const double* __restrict__ prims, const double* __restrict__ grad,
-                                                       const double* __restrict__ qbar, double dt, GasDev gas, double* __restrict__ face_bar) {
-    constexpr int V = D + 2, GS = grad_stride<D>();
+__global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_faces_adjoint(int faces, const FaceRow<double>* __restrict__ face_rows,
+                                                                          const double* __restrict__ wg, const double* __restrict__ qbar, double dt,
+                                                                          GasDev gas, double* __restrict__ face_bar) {
+    constexpr int V = D + 2, B = bar_stride<D>();
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= m.f) return;
-    double a[D];
-#pragma unroll
-    for (int k = 0; k < D; ++k) a[k] = m.area[D * f + k];
-    const double magnitude = sqrt(dot<D>(a, a));
+    if (f >= faces) return;
+    FaceRow<double> r;
+    load_face_row<double>(face_rows + f, r);
     double Lbar[V], Rbar[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) Lbar[v] = Rbar[v] = 0;
-    if (magnitude != 0) {
-        const int o = m.owner[f], j = m.neighbour[f];
-        double ro[D], rj[D], L[V], R[V], Wo[V], Wj[V], go[V * D], gj[V * D], n[D], Fbar[V];
-        m.face_offset(f, o, ro);
-        m.face_offset(f, j, rj);
+    if (r.mag != 0) {
+        double L[V], R[V], Fbar[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v)
+            Fbar[v] = r.mag * dt * (qbar[V * static_cast<int64_t>(r.j) + v] - qbar[V * static_cast<int64_t>(r.o) + v]);
+        {
+            double W[V], g[V * D];
+            load_wg<D>(wg, r.o, W, g);
+            side_value<D>(W, g, r.offo, dt, gas.gamma, L);
+        }
+        {
+            double W[V], g[V * D];
+            load_wg<D>(wg, r.j, W, g);
+            side_value<D>(W, g, r.offj, dt, gas.gamma, R);
+        }
+        if constexpr (Riemann == 1)
+            hll_flux_adjoint<D>(L, R, r.n, gas, Fbar, Lbar, Rbar);
+        else
+            hllc_flux_adjoint<D>(L, R, r.n, gas, Fbar, Lbar, Rbar);
+    }
+    double* row = face_bar + 2 * B * static_cast<int64_t>(f);
+    store_bar<V>(row, Lbar);
+    store_bar<V>(row + B, Rbar);
+}
+
+// AdjointCell (finite_volume.hpp:2107-2169), one thread a cell in the tiles' order (its entry rows are coalesced). The
+// half step's adjoint is linear in its bar, and a cell's sides differ only in r: the bars are summed over the faces first
+// and it is applied once.
+template <int D>
+__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_cell_adjoint(MeshDev<D> m, GeometryDev<D, double> geo,
+                                                                                const double* __restrict__ wg, double* face_bar,
+                                                                                const double* __restrict__ fit, const int32_t* __restrict__ clip,
+                                                                                double dt, GasDev gas, double* __restrict__ wbar) {
+    constexpr int V = D + 2, P = D + 1, B = bar_stride<D>();
+    using FL = FitLayout<D>;
+    const int64_t t = static_cast<int64_t>(blockIdx.x) * kTileCells + threadIdx.x;
+    const int i = geo.order[t];
+    if (i < 0) return;
+    const int first = m.start[i], count = m.start[i + 1] - first;
+    const int64_t slot0 = static_cast<int64_t>(geo.slice_base[t >> 5]) * 32 + (t & 31);
+    double Wi[V], Wi_bar[V], gi_bar[V * D];
+    {
+        double gi[V * D], half[V], S[V];  // S: the bars of the sides that did not fall back, summed
+        load_wg<D>(wg, i, Wi, gi);
+        half_step_rate<D, double>(Wi, gi, gas.gamma, half);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            Wo[v] = prims[PS * o + v];
-            Wj[v] = prims[PS * j + v];
+            half[v] = Wi[v] - 0.5 * dt * half[v];
+            Wi_bar[v] = S[v] = 0;
         }
 #pragma unroll
-        for (int c = 0; c < V * D; ++c) {
-            go[c] = grad[static_cast<int64_t>(GS) * o + c];
-            gj[c] = grad[static_cast<int64_t>(GS) * j + c];
+        for (int c = 0; c < V * D; ++c) gi_bar[c] = 0;
+        for (int k = 0; k < count; ++k) {
+            const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
+            const int32_t e = m.list[first + k];
+            double mb[V], r[D];
+            load_bar<V>(face_bar + B * (2 * static_cast<int64_t>(list_face(e)) + (e >= 0 ? 0 : 1)), mb);
+            const double2 o01 = geo.off01[slot];
+            r[0] = o01.x;
+            r[1] = o01.y;
+            if constexpr (D == 3) r[2] = geo.off2[slot];
+            const bool fallback = !(half[0] + dot<D>(gi, r) > 0 && half[P] + dot<D>(gi + D * P, r) > 0);  // side_value
+            if (fallback) {
+#pragma unroll
+                for (int v = 0; v < V; ++v) Wi_bar[v] += mb[v];
+            } else {
+#pragma unroll
+                for (int v = 0; v < V; ++v) {
+                    S[v] += mb[v];
+#pragma unroll
+                    for (int q = 0; q < D; ++q) gi_bar[D * v + q] += r[q] * mb[v];
+                }
+            }
         }
-        side_value<D>(Wo, go, ro, dt, gas.gamma, L);
-        side_value<D>(Wj, gj, rj, dt, gas.gamma, R);
-#pragma unroll
-        for (int v = 0; v < V; ++v) Fbar[v] = magnitude * dt * (qbar[V * j + v] - qbar[V * o + v]);
-        const double inv = 1.0 / magnitude;
-#pragma unroll
-        for (int k = 0; k < D; ++k) n[k] = a[k] * inv;
-        if constexpr (Riemann == 1)
-            hll_flux_adjoint<D>(L, R, n, gas, Fbar, Lbar, Rbar);
-        else
-            hllc_flux_adjoint<D>(L, R, n, gas, Fbar, Lbar, Rbar);
-    }
-    double* row = face_bar + 2 * V * static_cast<int64_t>(f);
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        row[v] = Lbar[v];
-        row[V + v] = Rbar[v];
-    }
-}
-
-// AdjointCell (finite_volume.hpp:2107-2169).
-template <int D>
-__global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_cell_adjoint(MeshDev<D> m, const double* __restrict__ prims, const double* __restrict__ grad,
-                                                      const double* __restrict__ face_bar, const double* __restrict__ fit,
-                                                      const int32_t* __restrict__ flags, double dt, GasDev gas, double* __restrict__ wbar,
-                                                      double* __restrict__ bbar, double* __restrict__ boundbar, int32_t* __restrict__ bound_face) {
-    constexpr int V = D + 2, U = D + 1, GS = grad_stride<D>();
-    using FL = FitLayout<D>;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.n) return;
-    double Wi[V], gi[V * D], Wi_bar[V], gi_bar[V * D];
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        Wi[v] = prims[PS * i + v];
-        Wi_bar[v] = 0;
-    }
-#pragma unroll
-    for (int c = 0; c < V * D; ++c) {
-        gi[c] = grad[static_cast<int64_t>(GS) * i + c];
-        gi_bar[c] = 0;
-    }
-    for (int k = m.start[i]; k < m.start[i + 1]; ++k) {
-        const int32_t e = m.list[k];
-        const int f = list_face(e);
-        double a[D];
-#pragma unroll
-        for (int q = 0; q < D; ++q) a[q] = m.area[D * f + q];
-        if (dot<D>(a, a) == 0) continue;
-        const double* mine = face_bar + 2 * V * static_cast<int64_t>(f) + (e >= 0 ? 0 : V);
-        double r[D], Wf[V], mb[V];
-        m.face_offset(f, i, r);
-#pragma unroll
-        for (int v = 0; v < V; ++v) mb[v] = mine[v];
-        if (side_value<D>(Wi, gi, r, dt, gas.gamma, Wf)) {
-#pragma unroll
-            for (int v = 0; v < V; ++v) Wi_bar[v] += mb[v];
-        } else {
-#pragma unroll
-            for (int v = 0; v < V; ++v)
-#pragma unroll
-                for (int q = 0; q < D; ++q) gi_bar[D * v + q] = gi_bar[D * v + q] + r[q] * mb[v];
-            half_step_adjoint<D>(Wi, gi, dt, gas.gamma, mb, Wi_bar, gi_bar);
-        }
+        half_step_adjoint<D>(Wi, gi, dt, gas.gamma, S, Wi_bar, gi_bar);
     }
     const double* fr = fit + static_cast<int64_t>(FL::width) * i;
-    double Lc[U][U];
+    double bound[V];
+    int bound_k[V];
 #pragma unroll
-    for (int p = 0; p < U; ++p)
+    for (int v = 0; v < V; ++v) {  // gi_bar becomes g0's bar
+        const int word = clip[V * static_cast<int64_t>(i) + v];
+        bound[v] = 0;
+        bound_k[v] = -1;
+        if ((word & 1) && (word & 4)) {
 #pragma unroll
-        for (int s = 0; s < U; ++s) Lc[p][s] = fr[FL::factor + p * U + s];
+            for (int a = 0; a < D; ++a) gi_bar[D * v + a] = 0;
+        } else if (word & 1) {
+            const int64_t slot = slot0 + 32 * static_cast<int64_t>(clip_entry(word));
+            double o[D], g0[D];
+            const double2 o01 = geo.off01[slot];
+            o[0] = o01.x;
+            o[1] = o01.y;
+            if constexpr (D == 3) o[2] = geo.off2[slot];
 #pragma unroll
-    for (int v = 0; v < V; ++v) {
-        const int flag = flags[2 * V * i + v];
-        double g0[D], g0bar[D], xbar[U], z[U], bs[U];
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-            g0[a] = fr[FL::g0 + D * v + a];
-            g0bar[a] = gi_bar[D * v + a];
-        }
-        double self = 0, bound = 0;
-        int face = -1;
-        if ((flag & 1) && (flag & 4)) {
-#pragma unroll
-            for (int a = 0; a < D; ++a) g0bar[a] = 0;
-        } else if (flag & 1) {
-            double o[D];
-#pragma unroll
-            for (int a = 0; a < D; ++a) o[a] = fr[FL::offset + D * v + a];
+            for (int a = 0; a < D; ++a) g0[a] = fr[FL::g0 + D * v + a];
             const double den = dot<D>(g0, o);
-            const double s = (fr[FL::bound + v] - Wi[v]) / den, t = dot<D>(gi_bar + D * v, g0) / den;
+            const double s = (fr[FL::bound + v] - Wi[v]) / den, tb = dot<D>(gi_bar + D * v, g0) / den;
 #pragma unroll
-            for (int a = 0; a < D; ++a) g0bar[a] = gi_bar[D * v + a] * s - o[a] * (s * t);
-            bound = t;
-            face = flags[2 * V * i + V + v];
-            self -= t;
+            for (int a = 0; a < D; ++a) gi_bar[D * v + a] = gi_bar[D * v + a] * s - o[a] * (s * tb);
+            bound[v] = tb;
+            bound_k[v] = bound_entry(word);
+            Wi_bar[v] -= tb;
         }
-        xbar[0] = 0;
-#pragma unroll
-        for (int a = 0; a < D; ++a) xbar[1 + a] = g0bar[a];
-        // solve_factored (finite_volume.hpp:688-702): b bar = M^-1 x bar
-#pragma unroll
-        for (int p = 0; p < U; ++p) {
-            double sum = xbar[p];
-#pragma unroll
-            for (int q = 0; q < p; ++q) sum -= Lc[p][q] * z[q];
-            z[p] = sum / Lc[p][p];
-        }
-#pragma unroll
-        for (int p = U - 1; p >= 0; --p) {
-            double sum = z[p];
-#pragma unroll
-            for (int q = p + 1; q < U; ++q) sum -= Lc[q][p] * bs[q];
-            bs[p] = sum / Lc[p][p];
-        }
-#pragma unroll
-        for (int p = 0; p < U; ++p) self -= fr[FL::row0 + p] * bs[p];
-        wbar[V * i + v] = Wi_bar[v] + self;
-#pragma unroll
-        for (int p = 0; p < U; ++p) bbar[static_cast<int64_t>(U * V) * i + U * v + p] = bs[p];
-        boundbar[V * i + v] = bound;
-        bound_face[V * i + v] = face;
     }
+    for (int k = 0; k < count; ++k) {
+        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
+        const int32_t e = m.list[first + k];
+        const double2 c01 = geo.c01[slot];
+        double c[D], share[V];
+        c[0] = c01.x;
+        c[1] = c01.y;
+        if constexpr (D == 3) c[2] = geo.c2[slot];
+#pragma unroll
+        for (int v = 0; v < V; ++v) {
+            share[v] = dot<D>(c, gi_bar + D * v);
+            Wi_bar[v] -= share[v];
+            if (k == bound_k[v]) share[v] += bound[v];
+        }
+        store_bar<V>(face_bar + B * (2 * static_cast<int64_t>(list_face(e)) + (e >= 0 ? 0 : 1)), share);
+    }
+#pragma unroll
+    for (int v = 0; v < V; ++v) wbar[V * static_cast<int64_t>(i) + v] = Wi_bar[v];
 }
 
-// AdjointGather (finite_volume.hpp:2171-2195): Qbar_j += primitive_adjoint(W_j bar) / V_j.
+// AdjointGather (finite_volume.hpp:2171-2195): Qbar_j += primitive_adjoint(W_j bar) / V_j, W_j's bar its own and its
+// neighbours' shares, from the other side of each of its faces' rows.
 template <int D>
 __global__ void __launch_bounds__(128) k_gather_adjoint(MeshDev<D> m, const double* __restrict__ q, const double* __restrict__ wbar,
-                                                        const double* __restrict__ bbar, const double* __restrict__ boundbar,
-                                                        const int32_t* __restrict__ bound_face, GasDev gas, double* __restrict__ qbar) {
-    constexpr int V = D + 2, U = D + 1;
+                                                        const double* __restrict__ face_bar, GasDev gas, double* __restrict__ qbar) {
+    constexpr int V = D + 2, B = bar_stride<D>();
     const int j = blockIdx.x * blockDim.x + threadIdx.x;
     if (j >= m.n) return;
     double W_bar[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) W_bar[v] = wbar[V * j + v];
-    double cj[D];
-#pragma unroll
-    for (int a = 0; a < D; ++a) cj[a] = m.cen[D * j + a];
-    constexpr int B = LUNA_ADJ_GATHER_BATCH;
+    for (int v = 0; v < V; ++v) W_bar[v] = wbar[V * static_cast<int64_t>(j) + v];
+    constexpr int kBatch = 4;  // rows requested together
     const int first = m.start[j], end = m.start[j + 1];
-    for (int k0 = first; k0 < end; k0 += B) {
-        int f[B], i[B];
+    for (int k0 = first; k0 < end; k0 += kBatch) {
+        int32_t e[kBatch];
+        double share[kBatch][V];
 #pragma unroll
-        for (int b = 0; b < B; ++b) {
-            const int32_t e = k0 + b < end ? m.list[k0 + b] : 0;
-            f[b] = list_face(e);
-            i[b] = k0 + b < end ? (e >= 0 ? m.neighbour[f[b]] : m.owner[f[b]]) : j;
-        }
+        for (int b = 0; b < kBatch; ++b) e[b] = k0 + b < end ? m.list[k0 + b] : 0;
 #pragma unroll
-        for (int b = 0; b < B; ++b) {
-            if (k0 + b >= end) break;
-            double sep[D], between[D];
-            m.separation(i[b], j, sep);
+        for (int b = 0; b < kBatch; ++b)
+            if (k0 + b < end) load_bar<V>(face_bar + B * (2 * static_cast<int64_t>(list_face(e[b])) + (e[b] >= 0 ? 1 : 0)), share[b]);
 #pragma unroll
-            for (int a = 0; a < D; ++a) between[a] = sep[a] + cj[a] - m.cen[D * i[b] + a];
-            const double w = m.mag[f[b]];
+        for (int b = 0; b < kBatch; ++b)
+            if (k0 + b < end)
 #pragma unroll
-            for (int v = 0; v < V; ++v) {
-                const double* bb = bbar + static_cast<int64_t>(U * V) * i[b] + U * v;
-                double sum = bb[0];
-#pragma unroll
-                for (int p = 1; p < U; ++p) sum += between[p - 1] * bb[p];
-                W_bar[v] += w * sum + (bound_face[V * i[b] + v] == f[b] ? boundbar[V * i[b] + v] : 0.0);
-            }
-        }
+                for (int v = 0; v < V; ++v) W_bar[v] += share[b][v];
     }
     const double inv = 1.0 / m.vol[j];
     double Uj[V], U_bar[V];
 #pragma unroll
-    for (int v = 0; v < V; ++v) Uj[v] = q[V * j + v] * inv;
+    for (int v = 0; v < V; ++v) Uj[v] = q[V * static_cast<int64_t>(j) + v] * inv;
     primitive_adjoint<D>(Uj, W_bar, gas, U_bar);
 #pragma unroll
-    for (int v = 0; v < V; ++v) qbar[V * j + v] += U_bar[v] * inv;
+    for (int v = 0; v < V; ++v) qbar[V * static_cast<int64_t>(j) + v] += U_bar[v] * inv;
 }
 
 }  // namespace luna

@@ -129,10 +129,11 @@ struct luna_fv {
     const float* mlp_params = nullptr;
     bool learned_inputs = false, apply_learned = false;
     // adjoint (allocated by the first luna_fv_step_adjoint)
-    DevArray<double> adj_fit, adj_face_bar, adj_wbar, adj_bbar, adj_boundbar, adj_qbar;
-    // tangent (allocated by the first luna_fv_step_tangent): dW, dg per cell, dF per face, a device copy of dq
+    DevArray<double> adj_fit, adj_face_bar, adj_wbar, adj_qbar;
+    DevArray<int32_t> adj_clip;
+    // tangent (allocated by the first luna_fv_step_tangent): dW and merged dW, dg rows per cell, dF per face, a device
+    // copy of dq
     DevArray<double> tan_dprims, tan_dgrad, tan_dflux, tan_dq;
-    DevArray<int32_t> adj_flags, adj_bound_face;
     // the order-0 moving step's derivatives (allocated by their first call): W and c_s rows and their tangents, w, dw, the
     // faces' dG or bar rows, the angle faces' bars, and device copies of the caller's host arrays
     DevArray<double> mv_W, mv_dW, mv_w, mv_dw, mv_face, mv_angle_Abar, mv_angle_dbar, mv_in[6];
@@ -987,52 +988,34 @@ luna_status moving_end(luna_fv* fv) {
     return LUNA_OK;
 }
 
+template <int D>
+luna_status run_fit(luna_fv* fv);
+
 // step_adjoint (finite_volume.hpp:2201-2231): the forward recompute (primitives, the sweep keeping its fit), then the
 // faces' Riemann adjoints, the cells' adjoints and the gather into Qbar.
 template <int D>
 luna_status run_adjoint(luna_fv* fv, double dt, double* qbar) {
-    fv->grads_in_wg = false;  // k_sweep_fit writes grad64
-    constexpr int V = D + 2, U = D + 1;
-    using FL = luna::FitLayout<D>;
+    constexpr int V = D + 2;
     const size_t N = static_cast<size_t>(fv->n), F = static_cast<size_t>(fv->f);
-    LUNA_TRY(fv->adj_fit.alloc(N * FL::width, "adjoint fit rows"));
-    LUNA_TRY(fv->adj_flags.alloc(N * 2 * V, "adjoint flags"));
-    LUNA_TRY(fv->adj_face_bar.alloc(F > 0 ? F * 2 * V : 1, "adjoint face bars"));
+    LUNA_TRY(fv->adj_face_bar.alloc(F > 0 ? F * 2 * luna::bar_stride<D>() : 1, "adjoint face bars"));
     LUNA_TRY(fv->adj_wbar.alloc(N * V, "adjoint W bars"));
-    LUNA_TRY(fv->adj_bbar.alloc(N * V * U, "adjoint b bars"));
-    LUNA_TRY(fv->adj_boundbar.alloc(N * V, "adjoint bound bars"));
-    LUNA_TRY(fv->adj_bound_face.alloc(N * V, "adjoint bound faces"));
+    LUNA_TRY(run_fit<D>(fv));
     const auto m = fv->mesh_dev<D>();
-    LUNA_TRY(run_primitives<D>(fv));
-    {
-        const long timed_ = fv->open_timed(1);
-        if (fv->limiter == LUNA_LIMITER_NONE)
-            luna::k_sweep_fit<D, false><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->adj_fit.ptr,
-                                                                                              fv->adj_flags.ptr);
-        else
-            luna::k_sweep_fit<D, true><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->adj_fit.ptr,
-                                                                                             fv->adj_flags.ptr);
-        fv->close_timed(timed_);
-    }
-    LUNA_CUDA(cudaGetLastError());
+    const auto geo = fv->geometry_dev<D, double>();
     if (F > 0) {
         const long timed_ = fv->open_timed(2);
-        if (fv->riemann == LUNA_HLL)
-            luna::k_faces_adjoint<D, 1><<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, qbar, dt, fv->gas,
-                                                                                              fv->adj_face_bar.ptr);
-        else
-            luna::k_faces_adjoint<D, 0><<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, qbar, dt, fv->gas,
-                                                                                              fv->adj_face_bar.ptr);
+        auto kernel = fv->riemann == LUNA_HLL ? luna::k_faces_adjoint<D, 1> : luna::k_faces_adjoint<D, 0>;
+        kernel<<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(static_cast<int>(F), geo.faces, fv->wg64.ptr, qbar, dt, fv->gas,
+                                                                       fv->adj_face_bar.ptr);
         fv->close_timed(timed_);
         LUNA_CUDA(cudaGetLastError());
     }
     {
         const long timed_ = fv->open_timed(3);
-        luna::k_cell_adjoint<D><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->adj_face_bar.ptr,
-                                                                                        fv->adj_fit.ptr, fv->adj_flags.ptr, dt, fv->gas, fv->adj_wbar.ptr,
-                                                                                        fv->adj_bbar.ptr, fv->adj_boundbar.ptr, fv->adj_bound_face.ptr);
-        luna::k_gather_adjoint<D><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->q.ptr, fv->adj_wbar.ptr, fv->adj_bbar.ptr,
-                                                                                          fv->adj_boundbar.ptr, fv->adj_bound_face.ptr, fv->gas, qbar);
+        luna::k_cell_adjoint<D><<<static_cast<unsigned int>(fv->tiles), luna::kTileCells, 0, fv->stream>>>(
+            m, geo, fv->wg64.ptr, fv->adj_face_bar.ptr, fv->adj_fit.ptr, fv->adj_clip.ptr, dt, fv->gas, fv->adj_wbar.ptr);
+        luna::k_gather_adjoint<D><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->q.ptr, fv->adj_wbar.ptr, fv->adj_face_bar.ptr,
+                                                                                          fv->gas, qbar);
         fv->close_timed(timed_);
     }
     LUNA_CUDA(cudaGetLastError());
@@ -1041,43 +1024,72 @@ luna_status run_adjoint(luna_fv* fv, double dt, double* qbar) {
     return LUNA_OK;
 }
 
+// launch(tiles, first tile, shared bytes) for a kernel of one block a tile that stages `row` doubles a staged cell: the
+// tiles within the row budget, then the others.
+template <class Launch>
+luna_status launch_tiles(luna_fv* fv, int row, const Launch& launch) {
+    const int64_t groups[2][2] = {{0, fv->normal_tiles}, {fv->normal_tiles, fv->tiles}};
+    const int most_rows[2] = {fv->normal_rows, fv->big_rows};
+    for (int k = 0; k < 2; ++k) {
+        const int64_t first = groups[k][0], count = groups[k][1] - groups[k][0];
+        if (count <= 0) continue;
+        launch(static_cast<unsigned int>(count), static_cast<int>(first), sizeof(double) * row * static_cast<size_t>(most_rows[k]));
+        LUNA_CUDA(cudaGetLastError());
+    }
+    return LUNA_OK;
+}
+
+// The derivatives' forward part: the primitive rows and the sweep with its fit kept, at the current state.
+template <int D>
+luna_status run_fit(luna_fv* fv) {
+    using FL = luna::FitLayout<D>;
+    const size_t N = static_cast<size_t>(fv->n);
+    LUNA_TRY(ensure_step_rows<D>(fv));
+    LUNA_TRY(fv->adj_fit.alloc(N * FL::width, "adjoint fit rows"));
+    LUNA_TRY(fv->adj_clip.alloc(N * (D + 2), "adjoint clip words"));
+    LUNA_TRY(run_primitives<D>(fv));
+    const auto m = fv->mesh_dev<D>();
+    const auto geo = fv->geometry_dev<D, double>();
+    const long timed_ = fv->open_timed(1);
+    auto kernel = fv->limiter == LUNA_LIMITER_NONE ? luna::k_sweep_fit<D, false> : luna::k_sweep_fit<D, true>;
+    const luna_status st = launch_tiles(fv, luna::kFitStaged, [&](unsigned int tiles, int first, size_t smem) {
+        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        kernel<<<tiles, luna::kTileCells, smem, fv->stream>>>(m, geo, first, fv->prims.ptr, fv->wg64.ptr, fv->adj_fit.ptr, fv->adj_clip.ptr);
+    });
+    fv->close_timed(timed_);
+    fv->grads_in_wg = true;
+    return st;
+}
+
 // step_tangent (finite_volume.hpp:2023-2062) before the step: dq <- J dq at fixed dt, linearised where step_adjoint is
-// (the reference's fit and clip pattern, k_sweep_fit), then the production step advances Q.
+// (k_sweep_fit's gradients and clip pattern), then the production step advances Q.
 template <int D>
 luna_status run_tangent(luna_fv* fv, double dt, double* dq) {
-    fv->grads_in_wg = false;  // k_sweep_fit writes grad64
     constexpr int V = D + 2;
-    using FL = luna::FitLayout<D>;
     const size_t N = static_cast<size_t>(fv->n), F = static_cast<size_t>(fv->f);
-    LUNA_TRY(fv->adj_fit.alloc(N * FL::width, "adjoint fit rows"));
-    LUNA_TRY(fv->adj_flags.alloc(N * 2 * V, "adjoint flags"));
-    LUNA_TRY(fv->tan_dprims.alloc(N * V, "tangent dW"));
-    LUNA_TRY(fv->tan_dgrad.alloc(N * V * D, "tangent dg"));
-    LUNA_TRY(fv->tan_dflux.alloc(F > 0 ? F * V : 1, "tangent dF"));
+    LUNA_TRY(fv->tan_dprims.alloc(N * luna::bar_stride<D>(), "tangent dW"));
+    LUNA_TRY(fv->tan_dgrad.alloc(N * luna::wg_stride<D>(), "tangent dW and dg rows"));
+    LUNA_TRY(fv->tan_dflux.alloc(F * V + 4, "tangent dF"));  // 4 doubles past the last row: load_row_windowed
+    LUNA_TRY(run_fit<D>(fv));
     const auto m = fv->mesh_dev<D>();
-    LUNA_TRY(run_primitives<D>(fv));
+    const auto geo = fv->geometry_dev<D, double>();
     {
         const long timed_ = fv->open_timed(1);
-        if (fv->limiter == LUNA_LIMITER_NONE)
-            luna::k_sweep_fit<D, false><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->adj_fit.ptr,
-                                                                                              fv->adj_flags.ptr);
-        else
-            luna::k_sweep_fit<D, true><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->adj_fit.ptr,
-                                                                                             fv->adj_flags.ptr);
         luna::k_tangent_prims<D><<<blocks(N, 256), 256, 0, fv->stream>>>(static_cast<int>(N), fv->q.ptr, dq, fv->vol.ptr, fv->gas, fv->tan_dprims.ptr);
-        luna::k_tangent_sweep<D><<<blocks(N, kBlockCells), kBlockCells, 0, fv->stream>>>(m, fv->prims.ptr, fv->tan_dprims.ptr, fv->adj_fit.ptr,
-                                                                                        fv->adj_flags.ptr, fv->tan_dgrad.ptr);
+        auto kernel = luna::k_tangent_sweep<D>;
+        const luna_status st = launch_tiles(fv, luna::kFitStaged, [&](unsigned int tiles, int first, size_t smem) {
+            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+            kernel<<<tiles, luna::kTileCells, smem, fv->stream>>>(m, geo, first, fv->tan_dprims.ptr, fv->wg64.ptr, fv->adj_fit.ptr, fv->adj_clip.ptr,
+                                                                  fv->tan_dgrad.ptr);
+        });
         fv->close_timed(timed_);
+        LUNA_TRY(st);
     }
-    LUNA_CUDA(cudaGetLastError());
     if (F > 0) {
         const long timed_ = fv->open_timed(2);
-        if (fv->riemann == LUNA_HLL)
-            luna::k_tangent_fluxes<D, 1><<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->tan_dprims.ptr,
-                                                                                               fv->tan_dgrad.ptr, dt, fv->gas, fv->tan_dflux.ptr);
-        else
-            luna::k_tangent_fluxes<D, 0><<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(m, fv->prims.ptr, fv->grad64.ptr, fv->tan_dprims.ptr,
-                                                                                               fv->tan_dgrad.ptr, dt, fv->gas, fv->tan_dflux.ptr);
+        auto kernel = fv->riemann == LUNA_HLL ? luna::k_tangent_fluxes<D, 1> : luna::k_tangent_fluxes<D, 0>;
+        kernel<<<blocks(F, kBlockFaces), kBlockFaces, 0, fv->stream>>>(static_cast<int>(F), geo.faces, fv->wg64.ptr, fv->tan_dgrad.ptr, dt, fv->gas,
+                                                                       fv->tan_dflux.ptr);
         fv->close_timed(timed_);
         LUNA_CUDA(cudaGetLastError());
     }
@@ -1088,7 +1100,7 @@ luna_status run_tangent(luna_fv* fv, double dt, double* dq) {
     }
     LUNA_CUDA(cudaGetLastError());
     fv->prims_ready = true;  // Q is unchanged
-    fv->swept = false;       // grad64 holds the fit's gradients: the step sweeps again
+    fv->swept = false;       // the merged rows hold the fit's gradients: the step sweeps again
     return LUNA_OK;
 }
 
@@ -1897,8 +1909,7 @@ LUNA_API luna_status luna_fv_device_bytes(luna_fv* fv, int64_t* out) {
     b += fv->q.bytes() + fv->next.bytes() + fv->prims.bytes() + fv->grad64.bytes() + fv->grad32.bytes() + fv->flux.bytes();
     b += fv->grad16.bytes() + fv->grad16_exp.bytes() + fv->wg64.bytes();
     b += fv->w.bytes() + fv->x.bytes() + fv->old_cen.bytes() + fv->steps.bytes() + fv->counters.bytes();
-    b += fv->adj_fit.bytes() + fv->adj_face_bar.bytes() + fv->adj_wbar.bytes() + fv->adj_bbar.bytes() + fv->adj_boundbar.bytes();
-    b += fv->adj_qbar.bytes() + fv->adj_flags.bytes() + fv->adj_bound_face.bytes();
+    b += fv->adj_fit.bytes() + fv->adj_face_bar.bytes() + fv->adj_wbar.bytes() + fv->adj_qbar.bytes() + fv->adj_clip.bytes();
     b += fv->tan_dprims.bytes() + fv->tan_dgrad.bytes() + fv->tan_dflux.bytes() + fv->tan_dq.bytes();
     b += fv->geo_c01.bytes() + fv->geo_c2.bytes() + fv->geo_off01.bytes() + fv->geo_off2.bytes() + fv->geo_nbr.bytes();
     b += fv->geo_slice_base.bytes() + fv->geo_order.bytes() + fv->geo_stage_start.bytes() + fv->geo_stage_cells.bytes() + fv->geo_faces.bytes();

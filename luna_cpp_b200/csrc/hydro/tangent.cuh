@@ -1,11 +1,11 @@
 // The tangent of one static step (luna-cpp's step_tangent, src/hydro/finite_volume.hpp:2023-2062): dQ^n+1 = J dQ^n at
 // fixed dt, for the FP64 policy, order 1, the per-face loop; the step itself runs after it with the production kernels,
-// so Q^n+1 is step()'s. The linearisation point is the adjoint's (k_sweep_fit: the reference's fit, its clip pattern and
-// gradients), so the tangent and the adjoint are transposes of one map (the dot test). Passes:
+// so Q^n+1 is step()'s. The linearisation point is the adjoint's (k_sweep_fit: its gradients and clip pattern), so the
+// tangent and the adjoint are transposes of one map (the dot test). Passes, over the step's own rows as the adjoint's:
 //   k_tangent_prims   dW = J dU of primitive() per cell (primitive_tangent, euler.hpp:131-142);
-//   k_tangent_sweep   dg per cell: the fit's tangent right-hand side over the list, solved with the stored Cholesky
-//                     factor, then the limited gradient's tangent at its clip pattern (limited_gradient_tangent,
-//                     finite_volume.hpp:811-833: a clipped variable is g0 (bound - W_i) / (g0 . o_last));
+//   k_tangent_sweep   dg per cell: dg0 = sum_k c_k (dW_k - dW_i) over the tile's staged dW, then the limited gradient's
+//                     tangent at its clip pattern (limited_gradient_tangent, finite_volume.hpp:811-833: a clipped
+//                     variable is g0 (bound - W_i) / (g0 . o_last)); merged rows dW, dg;
 //   k_tangent_fluxes  per face: both face states' tangents (side_tangent: the half step and g . r, a fallen-back side
 //                     carries dW) and the Riemann solve's, by forward-mode dual numbers through the same HLLC/HLL code
 //                     as the step (each branch the forward took), times |A| (TangentFluxes, :1971-2004);
@@ -122,14 +122,15 @@ __device__ __forceinline__ void primitive_tangent(const double* U, const double*
     dW[P] = (gas.gamma - 1.0) * de;
 }
 
+// dW rows of bar_stride doubles (what the tiles stage).
 template <int D>
 __global__ void __launch_bounds__(256) k_tangent_prims(int n, const double* __restrict__ q, const double* __restrict__ dq,
                                                        const double* __restrict__ vol, GasDev gas, double* __restrict__ dprims) {
-    constexpr int V = D + 2;
+    constexpr int V = D + 2, B = bar_stride<D>();
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const double inv = 1.0 / vol[i];
-    double U[V], dU[V], dW[V];
+    double U[V], dU[V], dW[B];
 #pragma unroll
     for (int v = 0; v < V; ++v) {
         U[v] = q[V * static_cast<int64_t>(i) + v] * inv;
@@ -137,98 +138,80 @@ __global__ void __launch_bounds__(256) k_tangent_prims(int n, const double* __re
     }
     primitive_tangent<D>(U, dU, gas, dW);
 #pragma unroll
-    for (int v = 0; v < V; ++v) dprims[V * static_cast<int64_t>(i) + v] = dW[v];
+    for (int v = V; v < B; ++v) dW[v] = 0;
+    store_bar<B>(dprims + B * static_cast<int64_t>(i), dW);
 }
 
-// The limited gradient's tangent per cell at the stored fit and clip pattern (k_sweep_fit's rows and flags).
+// The limited gradient's tangent per cell at the stored fit and clip pattern (k_sweep_fit's rows and clip words), one
+// block a tile.
 template <int D>
-__global__ void __launch_bounds__(128) k_tangent_sweep(MeshDev<D> m, const double* __restrict__ prims, const double* __restrict__ dprims,
-                                                       const double* __restrict__ fit, const int32_t* __restrict__ flags,
-                                                       double* __restrict__ dgrad) {
-    constexpr int V = D + 2, U = D + 1;
+__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_tangent_sweep(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
+                                                                                 const double* __restrict__ dprims, const double* __restrict__ wg,
+                                                                                 const double* __restrict__ fit, const int32_t* __restrict__ clip,
+                                                                                 double* __restrict__ dwg) {
+    constexpr int V = D + 2;
     using FL = FitLayout<D>;
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= m.n) return;
-    double dWi[V];
+    extern __shared__ double2 staged_rows[];
+    double* rows = reinterpret_cast<double*>(staged_rows);
+    const int tile = tile0 + static_cast<int>(blockIdx.x);
+    stage_rows<D>(geo, tile, dprims, bar_stride<D>(), rows);
+    const int64_t t = static_cast<int64_t>(tile) * kTileCells + threadIdx.x;
+    const int i = geo.order[t];
+    if (i < 0) return;
+    const int count = m.start[i + 1] - m.start[i];
+    const int64_t slot0 = static_cast<int64_t>(geo.slice_base[t >> 5]) * 32 + (t & 31);
+    double dWi[V], dg[V * D];
 #pragma unroll
-    for (int v = 0; v < V; ++v) dWi[v] = dprims[V * static_cast<int64_t>(i) + v];
-    double centroid[D];
+    for (int v = 0; v < V; ++v) dWi[v] = rows[kFitStaged * threadIdx.x + v];
 #pragma unroll
-    for (int a = 0; a < D; ++a) centroid[a] = m.cen[D * i + a];
-    double db[V][U];
-#pragma unroll
-    for (int v = 0; v < V; ++v)
-#pragma unroll
-        for (int p = 0; p < U; ++p) db[v][p] = 0;
-    for (int k = m.start[i]; k < m.start[i + 1]; ++k) {  // the fit's tangent right-hand side (limited_core, :733-737)
-        const int32_t e = m.list[k];
-        const int f = list_face(e);
-        const int j = e >= 0 ? m.neighbour[f] : m.owner[f];
-        double d[D], X[U];
-        m.separation(i, j, d);
-        X[0] = 1;
-#pragma unroll
-        for (int p = 1; p < U; ++p) X[p] = d[p - 1] + m.cen[D * j + p - 1] - centroid[p - 1];
-        const double w = m.mag[f];
+    for (int c = 0; c < V * D; ++c) dg[c] = 0;
+    for (int k = 0; k < count; ++k) {
+        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
+        const double2 c01 = geo.c01[slot];
+        double c[D], dWj[kFitStaged];
+        c[0] = c01.x;
+        c[1] = c01.y;
+        if constexpr (D == 3) c[2] = geo.c2[slot];
+        load_bar<V>(rows + kFitStaged * static_cast<int>(geo.nbr[slot] & kIndexMask), dWj);
 #pragma unroll
         for (int v = 0; v < V; ++v) {
-            const double ddW = w * (dprims[V * static_cast<int64_t>(j) + v] - dWi[v]);
+            const double ddW = dWj[v] - dWi[v];
 #pragma unroll
-            for (int p = 0; p < U; ++p) db[v][p] += X[p] * ddW;
+            for (int a = 0; a < D; ++a) dg[D * v + a] += c[a] * ddW;
         }
     }
     const double* fr = fit + static_cast<int64_t>(FL::width) * i;
-    double Lc[U][U];
-#pragma unroll
-    for (int p = 0; p < U; ++p)
-#pragma unroll
-        for (int s = 0; s < U; ++s) Lc[p][s] = fr[FL::factor + p * U + s];
-    double* out = dgrad + static_cast<int64_t>(V * D) * i;
 #pragma unroll
     for (int v = 0; v < V; ++v) {
-        double z[U], x[U];  // solve_factored (:688-699)
+        const int word = clip[V * static_cast<int64_t>(i) + v];
+        if (!(word & 1)) continue;
+        if (word & 4) {
 #pragma unroll
-        for (int p = 0; p < U; ++p) {
-            double sum = db[v][p];
-#pragma unroll
-            for (int q = 0; q < p; ++q) sum -= Lc[p][q] * z[q];
-            z[p] = sum / Lc[p][p];
+            for (int a = 0; a < D; ++a) dg[D * v + a] = 0.0;
+            continue;
         }
+        const int64_t slot = slot0 + 32 * static_cast<int64_t>(clip_entry(word));
+        double o[D], g0[D];
+        const double2 o01 = geo.off01[slot];
+        o[0] = o01.x;
+        o[1] = o01.y;
+        if constexpr (D == 3) o[2] = geo.off2[slot];
 #pragma unroll
-        for (int p = U - 1; p >= 0; --p) {
-            double sum = z[p];
+        for (int a = 0; a < D; ++a) g0[a] = fr[FL::g0 + D * v + a];
+        const unsigned int holder = geo.nbr[slot0 + 32 * static_cast<int64_t>(bound_entry(word))] & kIndexMask;
+        const double dbound = rows[kFitStaged * static_cast<int>(holder) + v];
+        const double den = dot<D>(g0, o);
+        const double s = (fr[FL::bound + v] - wg[static_cast<int64_t>(wg_stride<D>()) * i + v]) / den;
+        const double ds = (dbound - dWi[v] - s * dot<D>(dg + D * v, o)) / den;
 #pragma unroll
-            for (int q = p + 1; q < U; ++q) sum -= Lc[q][p] * x[q];
-            x[p] = sum / Lc[p][p];
-        }
-        double dg0[D], g0[D], o[D];
-#pragma unroll
-        for (int a = 0; a < D; ++a) {
-            dg0[a] = x[1 + a];
-            g0[a] = fr[FL::g0 + D * v + a];
-            o[a] = fr[FL::offset + D * v + a];
-        }
-        const int flag = flags[2 * V * static_cast<int64_t>(i) + v];
-        if (!(flag & 1)) {
-#pragma unroll
-            for (int a = 0; a < D; ++a) out[D * v + a] = dg0[a];
-        } else if (flag & 4) {
-#pragma unroll
-            for (int a = 0; a < D; ++a) out[D * v + a] = 0.0;
-        } else {
-            // the bound came through face bf from its other cell
-            const int bf = flags[2 * V * static_cast<int64_t>(i) + V + v];
-            const int holder = m.owner[bf] == i ? m.neighbour[bf] : m.owner[bf];
-            const double dbound = dprims[V * static_cast<int64_t>(holder) + v];
-            const double den = dot<D>(g0, o);
-            const double s = (fr[FL::bound + v] - prims[PS * static_cast<int64_t>(i) + v]) / den;
-            const double ds = (dbound - dWi[v] - s * dot<D>(dg0, o)) / den;
-#pragma unroll
-            for (int a = 0; a < D; ++a) out[D * v + a] = dg0[a] * s + g0[a] * ds;
-        }
+        for (int a = 0; a < D; ++a) dg[D * v + a] = dg[D * v + a] * s + g0[a] * ds;
     }
+    store_wg<D>(dwg, i, dWi, dg);
 }
 
+#ifndef LUNA_TANGENT_MIN_BLOCKS
+#define LUNA_TANGENT_MIN_BLOCKS 3
+#endif
 // side_tangent (finite_volume.hpp:1346-1366): the face state's tangent, by duals through the half step; a side that
 // fell back (rho or P of the face state not positive) carries dW.
 template <int D>
@@ -256,37 +239,33 @@ __device__ __forceinline__ void side_tangent(const double* W, const double* dW, 
 }
 
 template <int D, int Riemann>
-__global__ void __launch_bounds__(128) k_tangent_fluxes(MeshDev<D> m, const double* __restrict__ prims, const double* __restrict__ grad,
-                                                        const double* __restrict__ dprims, const double* __restrict__ dgrad, double dt, GasDev gas,
-                                                        double* __restrict__ dflux) {
-    constexpr int V = D + 2, GS = grad_stride<D>();
+__global__ void __launch_bounds__(128, LUNA_TANGENT_MIN_BLOCKS) k_tangent_fluxes(int faces, const FaceRow<double>* __restrict__ face_rows,
+                                                                               const double* __restrict__ wg, const double* __restrict__ dwg,
+                                                                               double dt, GasDev gas, double* __restrict__ dflux) {
+    constexpr int V = D + 2;
     const int f = blockIdx.x * blockDim.x + threadIdx.x;
-    if (f >= m.f) return;
-    const double magnitude = m.mag[f];
+    if (f >= faces) return;
+    FaceRow<double> r;
+    load_face_row<double>(face_rows + f, r);
     double dF[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) dF[v] = 0;
-    if (magnitude != 0) {
-        const int o = m.owner[f], j = m.neighbour[f];
-        double ro[D], rj[D];
-        m.face_offset(f, o, ro);
-        m.face_offset(f, j, rj);
-        double L[V], R[V], dL[V], dR[V];
-        const double *Wo = prims + PS * static_cast<int64_t>(o), *Wj = prims + PS * static_cast<int64_t>(j);
-        const double *go = grad + static_cast<int64_t>(GS) * o, *gj = grad + static_cast<int64_t>(GS) * j;
-        const bool fo = side_value<D>(Wo, go, ro, dt, gas.gamma, L), fj = side_value<D>(Wj, gj, rj, dt, gas.gamma, R);
-        side_tangent<D>(Wo, dprims + V * static_cast<int64_t>(o), go, dgrad + static_cast<int64_t>(V * D) * o, ro, dt, gas.gamma, fo, dL);
-        side_tangent<D>(Wj, dprims + V * static_cast<int64_t>(j), gj, dgrad + static_cast<int64_t>(V * D) * j, rj, dt, gas.gamma, fj, dR);
+    if (r.mag != 0) {
         fwd::Dual Ld[V], Rd[V], n[D], w[D], F[V];
-        const double inv = 1.0 / magnitude;
+        const auto side = [&](int i, const double* off, fwd::Dual* out) {
+            double W[V], g[V * D], dW[V], dg[V * D], Wf[V], dWf[V];
+            load_wg<D>(wg, i, W, g);
+            load_wg<D>(dwg, i, dW, dg);
+            const bool fallback = side_value<D>(W, g, off, dt, gas.gamma, Wf);
+            side_tangent<D>(W, dW, g, dg, off, dt, gas.gamma, fallback, dWf);
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            Ld[v] = fwd::Dual(L[v], dL[v]);
-            Rd[v] = fwd::Dual(R[v], dR[v]);
-        }
+            for (int v = 0; v < V; ++v) out[v] = fwd::Dual(Wf[v], dWf[v]);
+        };
+        side(r.o, r.offo, Ld);
+        side(r.j, r.offj, Rd);
 #pragma unroll
         for (int a = 0; a < D; ++a) {
-            n[a] = fwd::Dual(m.area[D * static_cast<int64_t>(f) + a] * inv);
+            n[a] = fwd::Dual(r.n[a]);
             w[a] = fwd::Dual(0.0);
         }
         if constexpr (Riemann == 1)
@@ -294,12 +273,13 @@ __global__ void __launch_bounds__(128) k_tangent_fluxes(MeshDev<D> m, const doub
         else
             hllc_flux<D, fwd::Dual>(Ld, Rd, n, w, fwd::Dual(gas.gamma), fwd::Dual(gas.inverse_gm1), F, false);
 #pragma unroll
-        for (int v = 0; v < V; ++v) dF[v] = F[v].d * magnitude;
+        for (int v = 0; v < V; ++v) dF[v] = F[v].d * r.mag;
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) dflux[V * static_cast<int64_t>(f) + v] = dF[v];
 }
 
+// Flux rows as k_update reads them (load_row_windowed: the buffer extends 24 B past its last row).
 template <int D>
 __global__ void __launch_bounds__(256) k_tangent_update(MeshDev<D> m, double* __restrict__ dq, const double* __restrict__ dflux, double dt) {
     constexpr int V = D + 2;
@@ -308,12 +288,23 @@ __global__ void __launch_bounds__(256) k_tangent_update(MeshDev<D> m, double* __
     double dsum[V];
 #pragma unroll
     for (int v = 0; v < V; ++v) dsum[v] = 0;
-    for (int k = m.start[i]; k < m.start[i + 1]; ++k) {
-        const int32_t e = m.list[k];
-        const double sign = e >= 0 ? 1.0 : -1.0;
-        const double* r = dflux + V * static_cast<int64_t>(list_face(e));
+    const int first = m.start[i], end = m.start[i + 1];
+    constexpr int kBatch = 2;
+    for (int k0 = first; k0 < end; k0 += kBatch) {
+        int32_t e[kBatch];
+        double row[kBatch][V];
 #pragma unroll
-        for (int v = 0; v < V; ++v) dsum[v] += sign * r[v];
+        for (int b = 0; b < kBatch; ++b) e[b] = k0 + b < end ? m.list[k0 + b] : 0;
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b)
+            if (k0 + b < end) load_row_windowed<V>(dflux + V * static_cast<int64_t>(list_face(e[b])), row[b]);
+#pragma unroll
+        for (int b = 0; b < kBatch; ++b) {
+            if (k0 + b >= end) break;
+            const double sign = e[b] >= 0 ? 1.0 : -1.0;
+#pragma unroll
+            for (int v = 0; v < V; ++v) dsum[v] += sign * row[b][v];
+        }
     }
 #pragma unroll
     for (int v = 0; v < V; ++v) dq[V * static_cast<int64_t>(i) + v] = dq[V * static_cast<int64_t>(i) + v] - dt * dsum[v];
