@@ -403,11 +403,14 @@ __device__ __forceinline__ void store_half_row(const HalfRows& out, int i, const
 #define LUNA_CLIP_BATCH 4  // entries of the clip walk whose offset rows are requested together
 #endif
 // Limit: 0 none, 1 the plain face-centroid limiter, 2 the learned limiter's inputs (the gradient left unlimited).
-// KB: entries whose streamed rows are requested together. Launched with blocks of kTileCells threads over tiles [tile0, tile0 + gridDim.x) and the shared memory of the most
-// rows one of them stages (kStagedDoubles doubles a row).
-template <int D, bool Moving, bool Grad, class G, int Limit, int KB = LUNA_SWEEP_BATCH,
-          int MINB = sizeof(G) == sizeof(double) ? LUNA_SWEEP_MIN_BLOCKS : LUNA_SWEEP_MIN_BLOCKS_F>
-__global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, GeometryDev<D, G> geo, int tile0, const double* __restrict__ prims,
+// KB: entries whose streamed rows are requested together. L: threads a cell, the entries dealt to them in turn, their
+// sums, ranges and clip factors combined by shuffles (L > 1: not for Limit 2): a cell's chain is a quarter as long, for
+// meshes whose tiles leave SMs idle (16^3: the sweep 31 -> 16 us). Launched with blocks of L kTileCells
+// threads over tiles [tile0, tile0 + gridDim.x) and the shared memory of the most rows one of them stages
+// (kStagedDoubles doubles a row).
+template <int D, bool Moving, bool Grad, class G, int Limit, int L = 1, int KB = LUNA_SWEEP_BATCH,
+          int MINB = (L > 1) ? 1 : sizeof(G) == sizeof(double) ? LUNA_SWEEP_MIN_BLOCKS : LUNA_SWEEP_MIN_BLOCKS_F>
+__global__ void __launch_bounds__(kTileCells * L, MINB) k_sweep_tiles(MeshDev<D> m, GeometryDev<D, G> geo, int tile0, const double* __restrict__ prims,
                                                                G* __restrict__ grad_out, double* __restrict__ w_out, double courant,
                                                                double round_off2, Counters* __restrict__ ctr, LearnedInputs learned,
                                                                HalfRows half, double* __restrict__ wg_out) {
@@ -415,15 +418,17 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
     double* rows = reinterpret_cast<double*>(staged_rows);
     constexpr int V = D + 2, GS = grad_stride<D>(), R = kStagedDoubles;
     constexpr bool exact = sizeof(G) == sizeof(double);
+    static_assert(L == 1 || (Limit != 2 && 32 % L == 0), "threads a cell");
     const int tile = tile0 + static_cast<int>(blockIdx.x);
-    const int64_t t = static_cast<int64_t>(tile) * kTileCells + threadIdx.x;
+    const int in_tile = static_cast<int>(threadIdx.x) / L, sub = static_cast<int>(threadIdx.x) % L;  // the cell, the entries' share
+    const int64_t t = static_cast<int64_t>(tile) * kTileCells + in_tile;
     const int i = geo.order[t];
     const int count = i >= 0 ? m.start[i + 1] - m.start[i] : 0;
-    const int64_t row0 = static_cast<int64_t>(geo.slice_base[t >> 5]) * 32;  // the warp's first slot
+    const int64_t row0 = static_cast<int64_t>(geo.slice_base[t >> 5]) * 32;  // the slice's first slot
     const int64_t slot0 = row0 + (t & 31);
     const unsigned long long once = l2_evict_first();  // entry rows are read once per step
 #if LUNA_SWEEP_L2_PREFETCH
-    if ((threadIdx.x & 31) == 0) {  // the warp's walk-1 entry rows, on their way to L2 while the block stages
+    if ((in_tile & 31) == 0 && sub == 0) {  // the warp's walk-1 entry rows, on their way to L2 while the block stages
         const int64_t rows = geo.slice_base[(t >> 5) + 1] - geo.slice_base[t >> 5];
         if (rows > 0) {
             prefetch_l2(geo.nbr + row0, static_cast<unsigned int>(rows * 32 * sizeof(unsigned int)));
@@ -437,17 +442,18 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
     {
         const int s0 = geo.stage_start[tile], staged = geo.stage_start[tile + 1] - s0;
         constexpr int kRowsInFlight = 4;
-        for (int r0 = 0; r0 < staged; r0 += kRowsInFlight * kTileCells) {
+        constexpr int kThreads = kTileCells * L;
+        for (int r0 = 0; r0 < staged; r0 += kRowsInFlight * kThreads) {
             int cell[kRowsInFlight];
 #pragma unroll
             for (int b = 0; b < kRowsInFlight; ++b) {
-                const int r = r0 + b * kTileCells + static_cast<int>(threadIdx.x);
+                const int r = r0 + b * kThreads + static_cast<int>(threadIdx.x);
                 cell[b] = r < staged ? geo.stage_cells[s0 + r] : -1;
             }
 #pragma unroll
             for (int b = 0; b < kRowsInFlight; ++b) {
                 if (cell[b] < 0) continue;
-                double* dst = rows + R * (r0 + b * kTileCells + static_cast<int>(threadIdx.x));
+                double* dst = rows + R * (r0 + b * kThreads + static_cast<int>(threadIdx.x));
                 const double* src = prims + PS * static_cast<int64_t>(cell[b]);
 #pragma unroll
                 for (int q = 0; q < 6; q += 2) cp_async16(dst + q, src + q);
@@ -462,7 +468,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
     double smallest_dt = 1.0e300;
     if (i >= 0) {
         // the cell's own row: tile cells are staged first, in thread order
-        const double* own = rows + R * threadIdx.x;
+        const double* own = rows + R * in_tile;
         double Wi[V];
 #pragma unroll
         for (int v = 0; v < V; ++v) Wi[v] = own[v];
@@ -496,13 +502,13 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
         // a cell instead of two a face (the same minimum, rounded once).
         double best_num = 1.0e300, best_den = 1.0;
         bool any_tiny = false;  // a face below 1e-6 of the surface (rare): walk 2 then reads the entry words again
-        for (int k0 = 0; k0 < count; k0 += kBatch) {
+        for (int k0 = sub; k0 < count; k0 += L * kBatch) {
             unsigned int word[kBatch];
             G c[kBatch][D];
 #pragma unroll
             for (int b = 0; b < kBatch; ++b) {
-                const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + b);
-                if (k0 + b < count) {
+                const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + L * b);
+                if (k0 + L * b < count) {
                     word[b] = ldg_hint(geo.nbr + slot, once);
                     if constexpr (Grad) {
                         const Pair<G> c01 = ldg_hint(geo.c01 + slot, once);
@@ -514,7 +520,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
             }
 #pragma unroll
             for (int b = 0; b < kBatch; ++b) {
-                if (k0 + b >= count) break;
+                if (k0 + L * b >= count) break;
                 const bool owned = (word[b] & kOwnedBit) != 0, tiny_face = (word[b] & kTinyBit) != 0;
                 any_tiny = any_tiny || tiny_face;
                 const double* rj = rows + R * static_cast<int>(word[b] & kIndexMask);
@@ -563,7 +569,23 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                 }
             }
         }
-        if (best_num < 1.0e300) smallest_dt = courant * (best_num / best_den);
+        if constexpr (L > 1) {  // the cell's threads combine their shares (the cell's L lanes are here together)
+            const unsigned int lanes = ((1u << L) - 1u) << (threadIdx.x & 31u & ~static_cast<unsigned int>(L - 1));
+#pragma unroll
+            for (int o = 1; o < L; o <<= 1) {
+                if constexpr (Grad)
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        const G l = __shfl_xor_sync(lanes, lo[v], o), h = __shfl_xor_sync(lanes, hi[v], o);
+                        lo[v] = l < lo[v] ? l : lo[v];
+                        hi[v] = h > hi[v] ? h : hi[v];
+#pragma unroll
+                        for (int a = 0; a < D; ++a) g[D * v + a] += __shfl_xor_sync(lanes, g[D * v + a], o);
+                    }
+                any_tiny = __shfl_xor_sync(lanes, static_cast<int>(any_tiny), o) || any_tiny;
+            }
+        }
+        if (best_num < 1.0e300) smallest_dt = courant * (best_num / best_den);  // each thread's own share's
         const double ci = own_at(V), ri = own_at(V + 1);
         double wi[D];
 #pragma unroll
@@ -582,8 +604,9 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
 #pragma unroll
                 for (int a = 0; a < D; ++a) wi[a] = wi[a] + centroid[a] * s;
             }
+            if (sub == 0)
 #pragma unroll
-            for (int a = 0; a < D; ++a) w_out[D * i + a] = wi[a];
+                for (int a = 0; a < D; ++a) w_out[D * i + a] = wi[a];
         }
         {
             double rel[D];
@@ -618,7 +641,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                 }
             }
 #if LUNA_SWEEP_L2_PREFETCH >= 2
-            if constexpr (Limit != 0) {  // the warp's walk-2 offset rows, when a lane of it clips
+            if constexpr (Limit != 0 && L == 1) {  // the warp's walk-2 offset rows, when a lane of it clips
                 const unsigned int here = __activemask();
                 const unsigned int need = __ballot_sync(here, !round_off_only);
                 if (need && static_cast<int>(threadIdx.x & 31) == __ffs(here) - 1) {
@@ -673,7 +696,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                 }
                 write_learned_inputs<D>(learned, row, Wi, ci, ri, g, lo, hi, alpha);
             }
-            if constexpr (Limit == 1 && exact) if (!round_off_only) {
+            if constexpr (Limit == 1 && exact && L == 1) if (!round_off_only) {
                 // The clip (Sweep walk 2, finite_volume.hpp:538-565): each face in list order (tiny ones left out)
                 // scales a variable's gradient so that its face value stays in [lo, hi].
                 constexpr int kClipBatch = LUNA_CLIP_BATCH;
@@ -712,28 +735,28 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                     }
                 }
             }
-            if constexpr (Limit == 1 && !exact) if (!round_off_only) {
-                // The float policies' clip (the range is of differences, lo <= 0 <= hi) in its min-factor form
-                // (finite_volume.hpp:1008-1034): scaling g by each face's factor in list order ends at g times the
-                // smallest factor, since after a clip the face sits on its bound and a later face clips again only
-                // with a smaller one. Per variable the smallest room / |dp| over the faces is held as a fraction and
-                // compared by cross products: no division in the walk, one per clipped variable (measured: the
-                // grad32 sweep 0.91 -> 0.80 ms at 128^3; the FP64 sweep keeps the list-order form, which is faster
-                // there).
+            if constexpr (Limit == 1 && (!exact || L > 1)) if (!round_off_only) {
+                // The clip in its min-factor form (finite_volume.hpp:1008-1034), for the float policies (whose range is of
+                // differences, lo <= 0 <= hi) and for a cell dealt to several threads: scaling g by each face's factor in
+                // list order ends at g times the smallest factor, since after a clip the face sits on its bound and a
+                // later face clips again only with a smaller one. Per variable the smallest room / |dp| over the faces is
+                // held as a fraction and compared by cross products: no division in the walk, one per clipped variable
+                // (measured: the grad32 sweep 0.91 -> 0.80 ms at 128^3; one thread a cell in FP64 keeps the list-order
+                // form, which is faster there).
                 G best_num[V], best_den[V];
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
                     best_num[v] = G(1);
                     best_den[v] = G(1);
                 }
-                constexpr int kClipBatch = LUNA_CLIP_BATCH;
-                for (int k0 = 0; k0 < count; k0 += kClipBatch) {
+                constexpr int kClipBatch = L > 1 ? 2 : LUNA_CLIP_BATCH;
+                for (int k0 = sub; k0 < count; k0 += L * kClipBatch) {
                     unsigned int word[kClipBatch];
                     G rg[kClipBatch][D];
 #pragma unroll
                     for (int b = 0; b < kClipBatch; ++b) {
-                        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + b);
-                        if (k0 + b < count) {
+                        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + L * b);
+                        if (k0 + L * b < count) {
                             word[b] = any_tiny ? ldg_hint(geo.nbr + slot, once) : 0u;
                             const Pair<G> o01 = ldg_hint(geo.off01 + slot, once);
                             rg[b][0] = o01.x;
@@ -743,13 +766,21 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                     }
 #pragma unroll
                     for (int b = 0; b < kClipBatch; ++b) {
-                        if (k0 + b >= count) break;
+                        if (k0 + L * b >= count) break;
                         if (word[b] & kTinyBit) continue;
 #pragma unroll
                         for (int v = 0; v < V; ++v) {
                             const G dp = dot<D>(g + D * v, rg[b]);
-                            const G room = dp > G(0) ? hi[v] : -lo[v], size = fabs(dp);
-                            if (dp != G(0) && size > room) {  // the face value would leave the range
+                            G room, size = fabs(dp);
+                            bool out;  // the face value would leave the range
+                            if constexpr (exact) {
+                                out = dp > 0 ? Wi[v] + dp > hi[v] : dp < 0 && Wi[v] + dp < lo[v];
+                                room = dp > 0 ? hi[v] - Wi[v] : Wi[v] - lo[v];
+                            } else {
+                                room = dp > G(0) ? hi[v] : -lo[v];
+                                out = dp != G(0) && size > room;
+                            }
+                            if (out) {
                                 const G num = room > G(0) ? room : G(0);
                                 if (num * best_den[v] < best_num[v] * size) {
                                     best_num[v] = num;
@@ -758,6 +789,19 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                             }
                         }
                     }
+                }
+                if constexpr (L > 1) {
+                    const unsigned int lanes = ((1u << L) - 1u) << (threadIdx.x & 31u & ~static_cast<unsigned int>(L - 1));
+#pragma unroll
+                    for (int o = 1; o < L; o <<= 1)
+#pragma unroll
+                        for (int v = 0; v < V; ++v) {
+                            const G num = __shfl_xor_sync(lanes, best_num[v], o), den = __shfl_xor_sync(lanes, best_den[v], o);
+                            if (num * best_den[v] < best_num[v] * den) {
+                                best_num[v] = num;
+                                best_den[v] = den;
+                            }
+                        }
                 }
 #pragma unroll
                 for (int v = 0; v < V; ++v) {
@@ -768,6 +812,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                     }
                 }
             }
+            if (sub == 0) {
             bool stored = false;
             if constexpr (!exact)
                 if (half.rows) {
@@ -803,6 +848,7 @@ __global__ void __launch_bounds__(kTileCells, MINB) k_sweep_tiles(MeshDev<D> m, 
                     else
                         out[c / per] = make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
                 }
+            }
             }
         }
     }

@@ -669,8 +669,10 @@ __device__ __forceinline__ void update_cell(const MeshDev<D>& m, double* __restr
 #endif
 // FS = float: the rows of store_flux_row, one aligned vector load each, widened to double before the sum (the
 // reference's static_cast<double>(F(f, v)), finite_volume.hpp:1607).
-template <int D, bool NextPrims, bool Windowed = false, class FS = double>
-__global__ void __launch_bounds__(256, Windowed ? (sizeof(FS) == sizeof(float) ? LUNA_UPDATE_MIN_BLOCKS_F : LUNA_UPDATE_MIN_BLOCKS) : 1) k_update(MeshDev<D> m, double* __restrict__ q, const FS* __restrict__ flux, double dt,
+// Small: for meshes that leave SMs idle, eight rows together and blocks of 64.
+constexpr int kSmallUpdateBlock = 64;
+template <int D, bool NextPrims, bool Windowed = false, class FS = double, bool Small = false>
+__global__ void __launch_bounds__(Small ? kSmallUpdateBlock : 256, Small || !Windowed ? 1 : sizeof(FS) == sizeof(float) ? LUNA_UPDATE_MIN_BLOCKS_F : LUNA_UPDATE_MIN_BLOCKS) k_update(MeshDev<D> m, double* __restrict__ q, const FS* __restrict__ flux, double dt,
                                                 double* __restrict__ prims, GasDev gas, Counters* __restrict__ ctr) {
     constexpr int V = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -681,7 +683,7 @@ __global__ void __launch_bounds__(256, Windowed ? (sizeof(FS) == sizeof(float) ?
     const int first = m.start[i], end = m.start[i + 1];
     // kBatch entries at a time: their list words, then their flux rows, are all requested before any is used (the
     // gathers of a list are independent); the sums stay in list order.
-    constexpr int kBatch = Windowed ? (sizeof(FS) == sizeof(float) ? LUNA_UPDATE_BATCH_F : LUNA_UPDATE_BATCH) : 4;
+    constexpr int kBatch = Small ? 8 : Windowed ? (sizeof(FS) == sizeof(float) ? LUNA_UPDATE_BATCH_F : LUNA_UPDATE_BATCH) : 4;
     for (int k0 = first; k0 < end; k0 += kBatch) {
         int32_t e[kBatch];
 #pragma unroll

@@ -492,8 +492,8 @@ luna_status run_primitives(luna_fv* fv) {
 }
 
 // The sweep's launches: the tiles within the row budget, then (rare) the single-cell tiles that stage more rows.
-template <int D, bool Moving, bool Grad, class G, int Limit>
-luna_status launch_sweep_tiles(luna_fv* fv, G* grad, double courant) {
+template <int D, bool Moving, bool Grad, class G, int Limit, int L>
+luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
     const auto m = fv->mesh_dev<D>();
     const auto geo = fv->geometry_dev<D, G>();
     // compact rows when the factors are applied (a step); every cell's row when the inputs are read (training data)
@@ -501,7 +501,7 @@ luna_status launch_sweep_tiles(luna_fv* fv, G* grad, double courant) {
     const luna::LearnedInputs learned{reinterpret_cast<__nv_bfloat16*>(fv->lim_features.ptr), fv->lim_alpha.ptr,
                                       compact ? fv->lim_cells.ptr : nullptr, compact ? fv->lim_count.ptr : nullptr};
     if (Limit == 2 && compact) LUNA_CUDA(cudaMemsetAsync(fv->lim_count.ptr, 0, sizeof(unsigned int), fv->stream));
-    auto kernel = luna::k_sweep_tiles<D, Moving, Grad, G, Limit>;
+    auto kernel = luna::k_sweep_tiles<D, Moving, Grad, G, Limit, L>;
     const luna::HalfRows half{fv->precision == LUNA_GRAD16 ? fv->grad16.ptr : nullptr, fv->grad16_exp.ptr};
     // merged rows for the static per-face FP64 step (the learned limiter's mode scales plain gradient rows)
     double* const wg_out = (Grad && Limit != 2 && sizeof(G) == sizeof(double)) ? fv->wg64.ptr : nullptr;
@@ -515,11 +515,24 @@ luna_status launch_sweep_tiles(luna_fv* fv, G* grad, double courant) {
         if (count <= 0) continue;
         const size_t smem = sizeof(double) * luna::kStagedDoubles * static_cast<size_t>(most_rows[k]);
         if (smem > 48 * 1024) LUNA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
-        kernel<<<static_cast<unsigned int>(count), luna::kTileCells, smem, fv->stream>>>(m, geo, static_cast<int>(first), fv->prims.ptr, grad, fv->w.ptr,
-                                                                                        courant, round_off2, fv->counters.ptr, learned, half, wg_out);
+        kernel<<<static_cast<unsigned int>(count), luna::kTileCells * L, smem, fv->stream>>>(m, geo, static_cast<int>(first), fv->prims.ptr, grad,
+                                                                                            fv->w.ptr, courant, round_off2, fv->counters.ptr, learned,
+                                                                                            half, wg_out);
         LUNA_CUDA(cudaGetLastError());
     }
     return LUNA_OK;
+}
+
+// Four threads a cell while one thread a cell leaves SMs without a tile (148 tiles of 128 cells). Measured, a whole step in
+// us at one / four threads a cell, point blast and smooth wave: 16^3 74 / 59 and 68 / 57, 24^3 75 / 61 and 71 / 61, 32^3
+// 86 / 78 and 82 / 84, 40^3 107 / 107 and 105 / 127; 2D wave 128^2 48 / 43, 200^2 53 / 64. The update's batches of eight
+// rows likewise (k_update): 16^3 4 us, 40^3 -7 us.
+constexpr int64_t kFewCells = 148 * luna::kTileCells;
+template <int D, bool Moving, bool Grad, class G, int Limit>
+luna_status launch_sweep_tiles(luna_fv* fv, G* grad, double courant) {
+    if constexpr (Limit != 2)
+        if (fv->n <= kFewCells) return launch_sweep_lanes<D, Moving, Grad, G, Limit, 4>(fv, grad, courant);
+    return launch_sweep_lanes<D, Moving, Grad, G, Limit, 1>(fv, grad, courant);
 }
 
 template <int D, bool Moving, bool Grad, class G>
@@ -682,14 +695,19 @@ luna::FluxArgs<D, G> flux_args(luna_fv* fv, const G* grad, double dt) {
 }
 
 // apply()'s update of the library's flux rows (windowed double rows, or single's float rows).
+template <int D, bool NextPrims, class FS, bool Small>
+void launch_update_rows(luna_fv* fv, double dt) {
+    constexpr int kBlock = Small ? luna::kSmallUpdateBlock : 256;
+    luna::k_update<D, NextPrims, true, FS, Small><<<blocks(fv->n, kBlock), kBlock, 0, fv->stream>>>(
+        fv->mesh_dev<D>(), fv->q.ptr, reinterpret_cast<const FS*>(fv->flux.ptr), dt, fv->prims.ptr, fv->gas, fv->counters.ptr);
+}
 template <int D, bool NextPrims>
 void launch_update(luna_fv* fv, double dt) {
+    const bool small = fv->n <= kFewCells;
     if (float_flux(fv))
-        luna::k_update<D, NextPrims, true, float><<<blocks(fv->n, 256), 256, 0, fv->stream>>>(
-            fv->mesh_dev<D>(), fv->q.ptr, reinterpret_cast<const float*>(fv->flux.ptr), dt, fv->prims.ptr, fv->gas, fv->counters.ptr);
+        small ? launch_update_rows<D, NextPrims, float, true>(fv, dt) : launch_update_rows<D, NextPrims, float, false>(fv, dt);
     else
-        luna::k_update<D, NextPrims, true><<<blocks(fv->n, 256), 256, 0, fv->stream>>>(fv->mesh_dev<D>(), fv->q.ptr, fv->flux.ptr, dt, fv->prims.ptr,
-                                                                                      fv->gas, fv->counters.ptr);
+        small ? launch_update_rows<D, NextPrims, double, true>(fv, dt) : launch_update_rows<D, NextPrims, double, false>(fv, dt);
 }
 
 // The fused pass's plan for the current mesh (tiles.h build_tile_faces on the host, from the device arrays), its face
