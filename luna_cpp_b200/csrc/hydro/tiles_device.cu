@@ -7,7 +7,6 @@
 // offsets; a filling pass repeats the table and writes the tiles.
 #include <cuda_runtime.h>
 
-#include <climits>
 #include <cub/device/device_radix_sort.cuh>
 #include <cub/device/device_scan.cuh>
 #include <string>
@@ -78,10 +77,11 @@ struct Box3 {
 int nblocks(int64_t n, int per) { return static_cast<int>((n + per - 1) / per); }
 
 template <int D>
-__global__ void k_morton(int64_t n, const double* __restrict__ pos, Box3 box, uint64_t* __restrict__ keys, int32_t* __restrict__ cells) {
+__global__ void k_morton(int64_t n, const double* __restrict__ pos, Box3 box, uint32_t* __restrict__ keys, int32_t* __restrict__ cells) {
     const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    keys[i] = luna::morton_key(D, pos + D * i, box.s);
+    // the top 32 of the key's bits (10 levels and more a side: a tile is 128 cells): half the passes of the sort
+    keys[i] = static_cast<uint32_t>(luna::morton_key(D, pos + D * i, box.s) >> (D == 3 ? 31 : 32));
     cells[i] = static_cast<int32_t>(i);
 }
 
@@ -112,14 +112,16 @@ struct FillOut {
 
 // A tile's distinct list neighbours are kept in a shared-memory hash table (open addressing, linear probing): kHash
 // slots, at most kHashFill distinct neighbours (more send the mesh to the host cut, as a tile with too many entries does).
-constexpr int kHash = 4096;
-constexpr int kHashFill = 3072;
-__device__ __forceinline__ int hash_slot(int32_t x) { return static_cast<int>((static_cast<uint32_t>(x) * 2654435761u) >> 20); }
+constexpr int kHash = 2048;
+constexpr int kHashFill = 1536;
+__device__ __forceinline__ int hash_slot(int32_t x) { return static_cast<int>((static_cast<uint32_t>(x) * 2654435761u) >> 21); }
 
 // One tile: plan (Fill false) or fill (Fill true). Each cell's thread inserts its list's neighbours into the block's
-// table; a neighbour seen for the first time that is not a cell of the tile joins the halo. The plan counts the rows
-// (the tile's cells and the halo); the fill sorts the halo by cell index, stages the rows and gives each list entry its
-// neighbour's row (a binary search among the tile's cells, else a table lookup).
+// table; a neighbour seen for the first time that is not a cell of the tile joins the halo, and its staged row (the tile's
+// cells first, in thread order, then the halo as it came) goes into the table beside it. The plan counts the rows; the
+// fill stages them and looks each list entry's row up. (The halo's order varies from run to run, the sweep's results do
+// not: the staged rows are copies. Sorted by cell, in a table of 4,096 slots, the two passes took 1.36 and 0.55 ms at
+// 128^3.)
 template <bool Fill>
 __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int32_t* __restrict__ sorted_cells, MeshLists m, PlanOut plan,
                                                             FillOut fill) {
@@ -174,9 +176,13 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
             for (; probe < kHash; ++probe) {
                 const int32_t prev = atomicCAS(&key[h], -1, x);
                 if (prev == -1) {
-                    if (own_index(x) < 0) {
+                    const int o = own_index(x);
+                    if (o < 0) {
                         const int q = atomicAdd(&n_halo, 1);
                         if (q < kHashFill) halo[q] = x;
+                        row_of[h] = static_cast<int16_t>(n_own + q);
+                    } else {
+                        row_of[h] = static_cast<int16_t>(own_row[o]);
                     }
                     break;
                 }
@@ -206,32 +212,6 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
                 atomicMax(rows > luna::kDeviceTileRows ? &plan.ctr->big_rows : &plan.ctr->normal_rows, rows);
         }
     } else {
-        // the halo by cell index (bitonic, ascending)
-        int P = 1;
-        while (P < halo_n) P <<= 1;
-        for (int q = halo_n + k; q < P; q += C) halo[q] = INT_MAX;
-        __syncthreads();
-        for (int size = 2; size <= P; size <<= 1)
-            for (int stride = size >> 1; stride > 0; stride >>= 1) {
-                for (int q = k; q < P; q += C) {
-                    const int r = q ^ stride;
-                    if (r > q) {
-                        const int32_t a = halo[q], b = halo[r];
-                        if ((a > b) == ((q & size) == 0)) {
-                            halo[q] = b;
-                            halo[r] = a;
-                        }
-                    }
-                }
-                __syncthreads();
-            }
-        for (int q = k; q < halo_n; q += C) {  // each halo cell's row, in the table (x was inserted: found within kHash)
-            const int32_t x = halo[q];
-            int h = hash_slot(x);
-            for (int probe = 0; probe < kHash && key[h] != x; ++probe) h = (h + 1) & (kHash - 1);
-            if (key[h] == x) row_of[h] = static_cast<int16_t>(n_own + q);
-        }
-        __syncthreads();
         const int64_t u = fill.tile_pos[t];
         const int64_t s0 = fill.stage_start[u];
         const int32_t mine_cell = ordered[k];
@@ -244,15 +224,9 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
             const int first = m.start[mine_cell], count = m.start[mine_cell + 1] - first;
             for (int e = 0; e < count; ++e) {
                 const int32_t x = m.other(m.list[first + e]);
-                const int o = own_index(x);
-                int row;
-                if (o >= 0) {
-                    row = own_row[o];
-                } else {  // a row the tile check rejects if x were missing (it was inserted: found within kHash)
-                    int h = hash_slot(x);
-                    for (int probe = 0; probe < kHash && key[h] != x; ++probe) h = (h + 1) & (kHash - 1);
-                    row = key[h] == x ? row_of[h] : rows;
-                }
+                int h = hash_slot(x);  // (x was inserted: found within kHash; a row the tile check rejects if it were not)
+                for (int probe = 0; probe < kHash && key[h] != x; ++probe) h = (h + 1) & (kHash - 1);
+                const int row = key[h] == x ? row_of[h] : rows;
                 fill.local[slot0 + 32 * static_cast<int64_t>(e)] = static_cast<uint32_t>(row);
             }
         }
@@ -326,7 +300,7 @@ namespace luna {
 
 class DeviceTiler {
 public:
-    Buf<uint64_t> keys, keys_sorted;
+    Buf<uint32_t> keys, keys_sorted;
     Buf<int32_t> cells, cells_sorted, rows, slice_len, normal, big, normal_before, big_before, pos, rows_u, len_u, stage_start, slice_base;
     Buf<TileCounters> ctr;
     Buf<unsigned int> bad;
@@ -376,9 +350,8 @@ luna_status device_tiles_plan(DeviceTiler* d, int dim, int64_t n, const double* 
     else
         k_morton<2><<<nblocks(n, 256), 256, 0, s>>>(n, pos, b, d->keys.ptr, d->cells.ptr);
     TL_CUDA(cudaGetLastError());
-    const int key_bits = dim == 3 ? 63 : 64;
     TL_TRY(d->with_temp([&](void* tmp, size_t& bytes) {
-        return cub::DeviceRadixSort::SortPairs(tmp, bytes, d->keys.ptr, d->keys_sorted.ptr, d->cells.ptr, d->cells_sorted.ptr, n, 0, key_bits, s);
+        return cub::DeviceRadixSort::SortPairs(tmp, bytes, d->keys.ptr, d->keys_sorted.ptr, d->cells.ptr, d->cells_sorted.ptr, n, 0, 32, s);
     }));
     TL_CUDA(cudaMemsetAsync(d->ctr.ptr, 0, sizeof(TileCounters), s));
     k_tiles<false><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(n, d->cells_sorted.ptr, d->lists, PlanOut{d->rows.ptr, d->slice_len.ptr, d->ctr.ptr},
