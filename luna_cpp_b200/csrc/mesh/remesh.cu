@@ -6,10 +6,11 @@
 //   buckets   counts (atomics), an exclusive scan, a fill (atomics), then each bucket's items sorted by index;
 //   cells     each cell's faces, by neighbour, appended to one face buffer at an atomic cursor (a cell's faces stay
 //             together; where they land does not matter, every later pass addresses them through the cell);
-//   faces     per owner (the lower-numbered cell): its faces towards higher cells plus the faces higher cells saw and it
-//             missed (flipped into its frame); a scan gives the face numbers, a segment with flipped faces is re-sorted
-//             by neighbour;
-//   lists     per cell, every face it is a side of (f, or ~f where it is not the owner), sorted by neighbour.
+//   faces     per owner (the lower-numbered cell): its faces towards higher cells, numbered by a scan, and
+//   lists     per cell, every face it is a side of (f, or ~f where it is not the owner), by neighbour: a cell's records as
+//             they are (k_emit_lists). Where a higher cell sees a face that the lower one misses (degenerate vertices),
+//             the general passes (assemble_general): such faces flipped into the owner's frame, a segment with them
+//             re-sorted by neighbour, the lists filled and sorted.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_scan.cuh>
@@ -219,6 +220,82 @@ __device__ __forceinline__ bool has_face(const int64_t* first, const int32_t* co
     return lo < first[c] + count[c] && fj[lo] == j;
 }
 
+struct FaceOut {
+    int32_t* owner;
+    int32_t* neighbour;
+    double* area;
+    double* fcen;
+};
+
+// ---- The assembly of a mesh whose cells agree on their faces (every face seen from both its cells: all but meshes with
+// degenerate vertices): a cell's records, by neighbour, are its list, the ones towards higher cells its owned faces in
+// order, and the number of one that a lower cell owns is found in that cell's records. No atomics and no sorts; bound by
+// the records copied. 128^3: 0.7 ms (k_forward, the scans and k_emit_lists' 0.63) where the general passes take 4.6.
+
+// Each cell's owned faces (records towards higher cells) and its list's length.
+__global__ void k_forward(int64_t n, const int64_t* __restrict__ first, const int32_t* __restrict__ count, const int32_t* __restrict__ fj,
+                          int64_t* __restrict__ owned, int32_t* __restrict__ degree) {
+    const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
+    if (i > n) return;
+    if (i == n) {
+        owned[n] = 0;
+        degree[n] = 0;
+        return;
+    }
+    const int64_t f0 = first[i], end = f0 + count[i];
+    int64_t lo = f0, hi = end;
+    while (lo < hi) {  // the first record past i
+        const int64_t mid = (lo + hi) >> 1;
+        if (fj[mid] <= i)
+            lo = mid + 1;
+        else
+            hi = mid;
+    }
+    owned[i] = end - lo;
+    degree[i] = count[i];
+}
+
+// Faces and lists, kEmitLanes threads a cell (neighbouring lanes copy neighbouring records). *missing counts the faces
+// that a higher cell sees and the lower one does not (the mesh is then assembled by the general passes).
+constexpr int kEmitLanes = 8;
+template <int D>
+__global__ void k_emit_lists(int64_t n, const int64_t* __restrict__ first, const int32_t* __restrict__ count, const int32_t* __restrict__ fj,
+                             const double* __restrict__ fa, const double* __restrict__ fc, const int64_t* __restrict__ face_start,
+                             const int32_t* __restrict__ start, FaceOut out, int32_t* __restrict__ list, unsigned int* __restrict__ missing) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x, i = t / kEmitLanes;
+    if (i >= n) return;
+    const int64_t f0 = first[i], own0 = face_start[i];
+    const int m = count[i], back = m - static_cast<int>(face_start[i + 1] - own0), s0 = start[i];
+    for (int k = static_cast<int>(t % kEmitLanes); k < m; k += kEmitLanes) {
+        const int64_t r = f0 + k;
+        const int32_t j = fj[r];
+        if (k >= back) {
+            const int64_t f = own0 + k - back;
+            out.owner[f] = static_cast<int32_t>(i);
+            out.neighbour[f] = j;
+            for (int a = 0; a < D; ++a) {
+                out.area[D * f + a] = fa[D * r + a];
+                out.fcen[D * f + a] = fc[D * r + a];
+            }
+            list[s0 + k] = static_cast<int32_t>(f);
+        } else {
+            const int64_t end = first[j] + count[j], begin = end - (face_start[j + 1] - face_start[j]);
+            int64_t lo = begin, hi = end;
+            while (lo < hi) {
+                const int64_t mid = (lo + hi) >> 1;
+                if (fj[mid] < i)
+                    lo = mid + 1;
+                else
+                    hi = mid;
+            }
+            if (lo < end && fj[lo] == i)
+                list[s0 + k] = ~static_cast<int32_t>(face_start[j] + (lo - begin));
+            else
+                atomicAdd(missing, 1u);
+        }
+    }
+}
+
 // Per owner: its faces towards higher cells (fwd), and (flips) the faces higher cells saw that it missed.
 __global__ void k_count_owned(int64_t n, const int64_t* __restrict__ first, const int32_t* __restrict__ count,
                               const int32_t* __restrict__ fj, int32_t* __restrict__ fwd, int32_t* __restrict__ flips,
@@ -250,12 +327,6 @@ __global__ void k_segment_lengths(int64_t n, const int32_t* __restrict__ fwd, co
     length[i] = i < n ? static_cast<int64_t>(fwd[i]) + flips[i] : 0;
 }
 
-struct FaceOut {
-    int32_t* owner;
-    int32_t* neighbour;
-    double* area;
-    double* fcen;
-};
 
 template <int D>
 __global__ void k_emit(int64_t n, const int64_t* __restrict__ first, const int32_t* __restrict__ count,
@@ -415,7 +486,56 @@ struct luna_remesh {
 
     template <int D>
     luna_status build(int64_t n, const double* points, bool on_device, luna_mesh_desc* mesh, int64_t* inconsistent);
+    template <int D>
+    luna_status assemble_general(int64_t n, int64_t* faces_out, Counters* h_out);
+    template <int D>
+    luna_status reserve_faces(int64_t F) {
+        RM_TRY(owner.reserve(F, "owner"));
+        RM_TRY(neighbour.reserve(F, "neighbour"));
+        RM_TRY(area.reserve(F * D, "area"));
+        RM_TRY(fcen.reserve(F * D, "face_centroid"));
+        return list.reserve(2 * F, "cell_face");
+    }
 };
+
+// Faces and lists where some face is seen from one of its cells only: the lower cell owns it all the same.
+template <int D>
+luna_status luna_remesh::assemble_general(int64_t n, int64_t* faces_out, Counters* h_out) {
+    const int T = 256;
+    int64_t F = 0;
+    Counters h{};
+    RM_CUDA(cudaMemsetAsync(flips.ptr, 0, n * sizeof(int32_t), stream));
+    k_count_owned<<<grid_blocks(n, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, fwd.ptr, flips.ptr, counters.ptr);
+    k_segment_lengths<<<grid_blocks(n + 1, T), T, 0, stream>>>(n, fwd.ptr, flips.ptr, seg_length.ptr);
+    RM_CUDA(cudaGetLastError());
+    RM_TRY(exclusive_scan(static_cast<const int64_t*>(seg_length.ptr), face_start.ptr, n + 1));
+    RM_CUDA(cudaMemcpyAsync(&F, face_start.ptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
+    RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
+    RM_CUDA(cudaStreamSynchronize(stream));
+    if (2 * F >= (int64_t(1) << 31) - 1) return fail(LUNA_EINVAL, "luna_remesh_build: too many faces for int32 lists");
+    RM_TRY(reserve_faces<D>(F));
+    RM_TRY(key.reserve(2 * F, "list keys"));
+    const FaceOut faces{owner.ptr, neighbour.ptr, area.ptr, fcen.ptr};
+    RM_CUDA(cudaMemsetAsync(cursor.ptr, 0, n * sizeof(unsigned int), stream));
+    k_emit<D><<<grid_blocks(n, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, fa.ptr, fc.ptr, pos.ptr, box, face_start.ptr,
+                                                    fwd.ptr, cursor.ptr, faces);
+    k_sort_segments<D><<<grid_blocks(n, T), T, 0, stream>>>(n, face_start.ptr, flips.ptr, faces);
+    RM_CUDA(cudaGetLastError());
+
+    // lists, by neighbour
+    RM_CUDA(cudaMemsetAsync(degree.ptr, 0, (n + 1) * sizeof(int32_t), stream));
+    if (F > 0) k_degree<<<grid_blocks(F, T), T, 0, stream>>>(F, owner.ptr, neighbour.ptr, degree.ptr);
+    RM_CUDA(cudaGetLastError());
+    RM_TRY(exclusive_scan(static_cast<const int32_t*>(degree.ptr), start.ptr, n + 1));
+    RM_CUDA(cudaMemsetAsync(cursor.ptr, 0, n * sizeof(unsigned int), stream));
+    if (F > 0) k_list_fill<<<grid_blocks(F, T), T, 0, stream>>>(F, owner.ptr, neighbour.ptr, start.ptr, cursor.ptr, list.ptr, key.ptr);
+    k_list_sort<<<grid_blocks(n, T), T, 0, stream>>>(n, start.ptr, list.ptr, key.ptr);
+    RM_CUDA(cudaGetLastError());
+    RM_CUDA(cudaStreamSynchronize(stream));
+    *faces_out = F;
+    *h_out = h;
+    return LUNA_OK;
+}
 
 template <int D>
 luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, luna_mesh_desc* mesh, int64_t* inconsistent) {
@@ -494,40 +614,27 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
         capacity = h.faces + h.faces / 16;
     }
 
-    // faces, by owner then neighbour
-    RM_CUDA(cudaMemsetAsync(flips.ptr, 0, n * sizeof(int32_t), stream));
-    k_count_owned<<<grid_blocks(n, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, fwd.ptr, flips.ptr, counters.ptr);
-    k_segment_lengths<<<grid_blocks(n + 1, T), T, 0, stream>>>(n, fwd.ptr, flips.ptr, seg_length.ptr);
+    // faces, by owner then neighbour, and lists, by neighbour
+    k_forward<<<grid_blocks(n + 1, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, seg_length.ptr, degree.ptr);
     RM_CUDA(cudaGetLastError());
     RM_TRY(exclusive_scan(static_cast<const int64_t*>(seg_length.ptr), face_start.ptr, n + 1));
+    RM_TRY(exclusive_scan(static_cast<const int32_t*>(degree.ptr), start.ptr, n + 1));
     int64_t F = 0;
     RM_CUDA(cudaMemcpyAsync(&F, face_start.ptr + n, sizeof(int64_t), cudaMemcpyDeviceToHost, stream));
-    RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
     RM_CUDA(cudaStreamSynchronize(stream));
-    if (2 * F >= (int64_t(1) << 31) - 1) return fail(LUNA_EINVAL, "luna_remesh_build: too many faces for int32 lists");
-    RM_TRY(owner.reserve(F, "owner"));
-    RM_TRY(neighbour.reserve(F, "neighbour"));
-    RM_TRY(area.reserve(F * D, "area"));
-    RM_TRY(fcen.reserve(F * D, "face_centroid"));
-    RM_TRY(list.reserve(2 * F, "cell_face"));
-    RM_TRY(key.reserve(2 * F, "list keys"));
-    const FaceOut faces{owner.ptr, neighbour.ptr, area.ptr, fcen.ptr};
-    RM_CUDA(cudaMemsetAsync(cursor.ptr, 0, n * sizeof(unsigned int), stream));
-    k_emit<D><<<grid_blocks(n, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, fa.ptr, fc.ptr, pos.ptr, box, face_start.ptr,
-                                                    fwd.ptr, cursor.ptr, faces);
-    k_sort_segments<D><<<grid_blocks(n, T), T, 0, stream>>>(n, face_start.ptr, flips.ptr, faces);
-    RM_CUDA(cudaGetLastError());
-
-    // lists, by neighbour
-    RM_CUDA(cudaMemsetAsync(degree.ptr, 0, (n + 1) * sizeof(int32_t), stream));
-    if (F > 0) k_degree<<<grid_blocks(F, T), T, 0, stream>>>(F, owner.ptr, neighbour.ptr, degree.ptr);
-    RM_CUDA(cudaGetLastError());
-    RM_TRY(exclusive_scan(static_cast<const int32_t*>(degree.ptr), start.ptr, n + 1));
-    RM_CUDA(cudaMemsetAsync(cursor.ptr, 0, n * sizeof(unsigned int), stream));
-    if (F > 0) k_list_fill<<<grid_blocks(F, T), T, 0, stream>>>(F, owner.ptr, neighbour.ptr, start.ptr, cursor.ptr, list.ptr, key.ptr);
-    k_list_sort<<<grid_blocks(n, T), T, 0, stream>>>(n, start.ptr, list.ptr, key.ptr);
-    RM_CUDA(cudaGetLastError());
-    RM_CUDA(cudaStreamSynchronize(stream));
+    bool agreed = static_cast<unsigned long long>(2 * F) == h.faces && 2 * F < (int64_t(1) << 31) - 1;
+    if (agreed) {
+        RM_TRY(reserve_faces<D>(F));
+        RM_CUDA(cudaMemsetAsync(cursor.ptr, 0, sizeof(unsigned int), stream));
+        k_emit_lists<D><<<grid_blocks(n * kEmitLanes, T), T, 0, stream>>>(n, first.ptr, count.ptr, fj.ptr, fa.ptr, fc.ptr, face_start.ptr, start.ptr,
+                                                                          FaceOut{owner.ptr, neighbour.ptr, area.ptr, fcen.ptr}, list.ptr, cursor.ptr);
+        RM_CUDA(cudaGetLastError());
+        unsigned int missing = 0;
+        RM_CUDA(cudaMemcpyAsync(&missing, cursor.ptr, sizeof(missing), cudaMemcpyDeviceToHost, stream));
+        RM_CUDA(cudaStreamSynchronize(stream));
+        agreed = missing == 0;
+    }
+    if (!agreed) RM_TRY(assemble_general<D>(n, &F, &h));
 
     *mesh = luna_mesh_desc{};
     mesh->dim = D;
