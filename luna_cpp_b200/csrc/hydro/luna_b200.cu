@@ -503,8 +503,8 @@ luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
     if (Limit == 2 && compact) LUNA_CUDA(cudaMemsetAsync(fv->lim_count.ptr, 0, sizeof(unsigned int), fv->stream));
     auto kernel = luna::k_sweep_tiles<D, Moving, Grad, G, Limit, L>;
     const luna::HalfRows half{fv->precision == LUNA_GRAD16 ? fv->grad16.ptr : nullptr, fv->grad16_exp.ptr};
-    // merged rows for the static per-face FP64 step (the learned limiter's mode scales plain gradient rows)
-    double* const wg_out = (Grad && Limit != 2 && sizeof(G) == sizeof(double)) ? fv->wg64.ptr : nullptr;
+    // merged rows for the static per-face FP64 step (the learned limiter's inputs for training go with plain rows)
+    double* const wg_out = (Grad && (Limit != 2 || compact) && sizeof(G) == sizeof(double)) ? fv->wg64.ptr : nullptr;
     fv->grads_in_wg = wg_out != nullptr;
     const int64_t groups[2][2] = {{0, fv->normal_tiles}, {fv->normal_tiles, fv->tiles}};
     const int most_rows[2] = {fv->normal_rows, fv->big_rows};
@@ -563,8 +563,10 @@ luna_status launch_sweep(luna_fv* fv, G* grad, double courant) {
                     return st;
                 }
             }
-            luna::k_apply_factors<D><<<blocks(fv->n, 256), 256, 0, fv->stream>>>(static_cast<int>(fv->n), fv->lim_cells.ptr, fv->lim_count.ptr, grad,
-                                                                                 fv->lim_alpha.ptr, fv->lim_logits.ptr, fv->mlp_params != nullptr);
+            auto kernel = fv->grads_in_wg ? luna::k_apply_factors<D, true> : luna::k_apply_factors<D, false>;
+            kernel<<<blocks(fv->n, 128), 128, 0, fv->stream>>>(static_cast<int>(fv->n), fv->lim_cells.ptr, fv->lim_count.ptr,
+                                                               fv->grads_in_wg ? fv->wg64.ptr : grad, fv->lim_alpha.ptr, fv->lim_logits.ptr,
+                                                               fv->mlp_params != nullptr);
             fv->close_timed(timed_);
             LUNA_CUDA(cudaGetLastError());
         }
@@ -823,7 +825,7 @@ luna_status run_apply(luna_fv* fv, const G* grad, double dt) {
         return fv->riemann == LUNA_HLL ? launch_per_cell<D, 1, G, false, 1>(fv, x, dt) : launch_per_cell<D, 1, G, false, 0>(fv, x, dt);
     }
     if constexpr (sizeof(G) == sizeof(double)) {
-        if (fv->order == 1 && fv->grads_in_wg) {
+        if (fv->order == 1 && fv->grads_in_wg && !fv->learned_inputs) {
             if (fv->fused == 0) LUNA_TRY(plan_fused<D>(fv));
             if (fv->fused == 1) {
                 auto y = x;
@@ -853,7 +855,7 @@ template <int D>
 luna_status flux_ahead(luna_fv* fv, bool* ahead) {
     *ahead = false;
     if (fv->motion == LUNA_MOVING || fv->update != LUNA_UPDATE_PER_FACE) return LUNA_OK;
-    if (fv->precision == LUNA_FP64 && fv->order == 1 && fv->grads_in_wg) {
+    if (fv->precision == LUNA_FP64 && fv->order == 1 && fv->grads_in_wg && !fv->learned_inputs) {
         if (fv->fused == 0) LUNA_TRY(plan_fused<D>(fv));
         if (fv->fused == 1) return LUNA_OK;
     }
