@@ -392,6 +392,10 @@ __device__ __forceinline__ void store_half_row(const HalfRows& out, int i, const
 #ifndef LUNA_SWEEP_MIN_BLOCKS_F
 #define LUNA_SWEEP_MIN_BLOCKS_F LUNA_SWEEP_MIN_BLOCKS  // the float policies' sweep
 #endif
+#ifndef LUNA_SWEEP_MIN_BLOCKS_2D
+#define LUNA_SWEEP_MIN_BLOCKS_2D 5  // 2D (96 registers hold its four variables; an eight-step rollout of 512^2 with its
+                                    // sweeps back: 3.97 ms at 4, 3.87 at 5; 6 spills)
+#endif
 #ifndef LUNA_SWEEP_BATCH
 #define LUNA_SWEEP_BATCH 0  // 0: 2 entries in FP64, 3 in the float policies (128^3 sweep ms: FP64 2: 0.748, 1: 0.760,
                             // 3: 0.794; riemann32 3: 0.536, 2: 0.545)
@@ -409,7 +413,7 @@ __device__ __forceinline__ void store_half_row(const HalfRows& out, int i, const
 // threads over tiles [tile0, tile0 + gridDim.x) and the shared memory of the most rows one of them stages
 // (kStagedDoubles doubles a row).
 template <int D, bool Moving, bool Grad, class G, int Limit, int L = 1, int KB = LUNA_SWEEP_BATCH,
-          int MINB = (L > 1) ? 1 : sizeof(G) == sizeof(double) ? LUNA_SWEEP_MIN_BLOCKS : LUNA_SWEEP_MIN_BLOCKS_F>
+          int MINB = (L > 1) ? 1 : D == 2 ? LUNA_SWEEP_MIN_BLOCKS_2D : sizeof(G) == sizeof(double) ? LUNA_SWEEP_MIN_BLOCKS : LUNA_SWEEP_MIN_BLOCKS_F>
 __global__ void __launch_bounds__(kTileCells * L, MINB) k_sweep_tiles(MeshDev<D> m, GeometryDev<D, G> geo, int tile0, const double* __restrict__ prims,
                                                                G* __restrict__ grad_out, double* __restrict__ w_out, double courant,
                                                                double round_off2, Counters* __restrict__ ctr, LearnedInputs learned,
