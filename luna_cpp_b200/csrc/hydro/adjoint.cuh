@@ -430,15 +430,25 @@ __device__ __forceinline__ bool side_value(const double* W, const double* g, con
     return fallback;
 }
 
+// Resident blocks an SM the adjoint's register-heavy kernels are cut for; with it k_sweep_fit and k_cell_adjoint request
+// two entries' rows together. Measured (one entry at a time, 4 blocks in 2D too -> now): Jacobian products at 72 x 64 x 60
+// 1.95 -> 1.90 ms, an eight-step rollout of 512^2 and back 4.08 -> 3.87 ms.
 #ifndef LUNA_ADJ_MIN_BLOCKS
-#define LUNA_ADJ_MIN_BLOCKS 4  // resident blocks an SM the adjoint's register-heavy kernels are cut for
+#define LUNA_ADJ_MIN_BLOCKS 4  // in 3D
 #endif
+#ifndef LUNA_ADJ_MIN_BLOCKS_2D
+#define LUNA_ADJ_MIN_BLOCKS_2D 5
+#endif
+template <int D>
+constexpr int adj_min_blocks() {
+    return D == 3 ? LUNA_ADJ_MIN_BLOCKS : LUNA_ADJ_MIN_BLOCKS_2D;
+}
 
 // The sweep again with the fit kept (Sweep<false, true, SweepFitHook<false>>), one block a tile as k_sweep_tiles: the
 // merged rows W, g (limited in list order: no round-off rule, so that every clip is the reference's), the fit rows
 // [N][FitLayout::width] and the clip words [N][V].
 template <int D, bool Limit>
-__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
+__global__ void __launch_bounds__(kTileCells, adj_min_blocks<D>()) k_sweep_fit(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
                                                                              const double* __restrict__ prims, double* __restrict__ wg,
                                                                              double* __restrict__ fit, int32_t* __restrict__ clip) {
     constexpr int V = D + 2;
@@ -465,32 +475,43 @@ __global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(M
         for (int a = 0; a < D; ++a) g[D * v + a] = 0;
     }
     bool any_tiny = false;
-    for (int k = 0; k < count; ++k) {
-        const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
-        const unsigned int word = geo.nbr[slot];
-        const double2 c01 = geo.c01[slot];
-        double c[D];
-        c[0] = c01.x;
-        c[1] = c01.y;
-        if constexpr (D == 3) c[2] = geo.c2[slot];
-        const double* rj = rows + kFitStaged * static_cast<int>(word & kIndexMask);
-        double Wj[kFitStaged];
+    constexpr int kBatch = 2;  // entries whose rows are requested together
+    for (int k0 = 0; k0 < count; k0 += kBatch) {
+        unsigned int word[kBatch];
+        double c[kBatch][D];
 #pragma unroll
-        for (int q = 0; q < (D == 3 ? 6 : 4); q += 2) {
-            const double2 w2 = *reinterpret_cast<const double2*>(rj + q);
-            Wj[q] = w2.x;
-            Wj[q + 1] = w2.y;
+        for (int b = 0; b < kBatch; ++b) {
+            if (k0 + b >= count) continue;
+            const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + b);
+            word[b] = geo.nbr[slot];
+            const double2 c01 = geo.c01[slot];
+            c[b][0] = c01.x;
+            c[b][1] = c01.y;
+            if constexpr (D == 3) c[b][2] = geo.c2[slot];
         }
-        const bool tiny_face = (word & kTinyBit) != 0;
-        any_tiny = any_tiny || tiny_face;
 #pragma unroll
-        for (int v = 0; v < V; ++v) {
-            const double dW = Wj[v] - Wi[v];
+        for (int b = 0; b < kBatch; ++b) {
+            const int k = k0 + b;
+            if (k >= count) continue;
+            const double* rj = rows + kFitStaged * static_cast<int>(word[b] & kIndexMask);
+            double Wj[kFitStaged];
 #pragma unroll
-            for (int a = 0; a < D; ++a) g[D * v + a] += c[a] * dW;
-            if (!tiny_face) {  // neighbour_range (finite_volume.hpp:572-588) leaves the tiny faces out
-                if (Wj[v] < lo[v]) lo[v] = Wj[v], lo_k[v] = k;
-                if (Wj[v] > hi[v]) hi[v] = Wj[v], hi_k[v] = k;
+            for (int q = 0; q < (D == 3 ? 6 : 4); q += 2) {
+                const double2 w2 = *reinterpret_cast<const double2*>(rj + q);
+                Wj[q] = w2.x;
+                Wj[q + 1] = w2.y;
+            }
+            const bool tiny_face = (word[b] & kTinyBit) != 0;
+            any_tiny = any_tiny || tiny_face;
+#pragma unroll
+            for (int v = 0; v < V; ++v) {
+                const double dW = Wj[v] - Wi[v];
+#pragma unroll
+                for (int a = 0; a < D; ++a) g[D * v + a] += c[b][a] * dW;
+                if (!tiny_face) {  // neighbour_range (finite_volume.hpp:572-588) leaves the tiny faces out
+                    if (Wj[v] < lo[v]) lo[v] = Wj[v], lo_k[v] = k;
+                    if (Wj[v] > hi[v]) hi[v] = Wj[v], hi_k[v] = k;
+                }
             }
         }
     }
@@ -538,7 +559,7 @@ __global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_sweep_fit(M
 // AdjointFaces (finite_volume.hpp:2078-2102): per face, the bars of its two face states from Qbar's jump across it, into
 // the face's row of two sides.
 template <int D, int Riemann>
-__global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_faces_adjoint(int faces, const FaceRow<double>* __restrict__ face_rows,
+__global__ void __launch_bounds__(128, adj_min_blocks<D>()) k_faces_adjoint(int faces, const FaceRow<double>* __restrict__ face_rows,
                                                                           const double* __restrict__ wg, const double* __restrict__ qbar, double dt,
                                                                           GasDev gas, double* __restrict__ face_bar) {
     constexpr int V = D + 2, B = bar_stride<D>();
@@ -578,7 +599,7 @@ __global__ void __launch_bounds__(128, LUNA_ADJ_MIN_BLOCKS) k_faces_adjoint(int 
 // half step's adjoint is linear in its bar, and a cell's sides differ only in r: the bars are summed over the faces first
 // and it is applied once.
 template <int D>
-__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_cell_adjoint(MeshDev<D> m, GeometryDev<D, double> geo,
+__global__ void __launch_bounds__(kTileCells, adj_min_blocks<D>()) k_cell_adjoint(MeshDev<D> m, GeometryDev<D, double> geo,
                                                                                 const double* __restrict__ wg, double* face_bar,
                                                                                 const double* __restrict__ fit, const int32_t* __restrict__ clip,
                                                                                 double dt, GasDev gas, double* __restrict__ wbar) {
@@ -601,25 +622,36 @@ __global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_cell_adjoin
         }
 #pragma unroll
         for (int c = 0; c < V * D; ++c) gi_bar[c] = 0;
-        for (int k = 0; k < count; ++k) {
-            const int64_t slot = slot0 + 32 * static_cast<int64_t>(k);
-            const int32_t e = m.list[first + k];
-            double mb[V], r[D];
-            load_bar<V>(face_bar + B * (2 * static_cast<int64_t>(list_face(e)) + (e >= 0 ? 0 : 1)), mb);
-            const double2 o01 = geo.off01[slot];
-            r[0] = o01.x;
-            r[1] = o01.y;
-            if constexpr (D == 3) r[2] = geo.off2[slot];
-            const bool fallback = !(half[0] + dot<D>(gi, r) > 0 && half[P] + dot<D>(gi + D * P, r) > 0);  // side_value
-            if (fallback) {
+        constexpr int kBatch = 2;  // entries whose rows are requested together
+        for (int k0 = 0; k0 < count; k0 += kBatch) {
+            int32_t e[kBatch];
+            double mb[kBatch][V], r[kBatch][D];
 #pragma unroll
-                for (int v = 0; v < V; ++v) Wi_bar[v] += mb[v];
-            } else {
+            for (int b = 0; b < kBatch; ++b) e[b] = k0 + b < count ? m.list[first + k0 + b] : 0;
 #pragma unroll
-                for (int v = 0; v < V; ++v) {
-                    S[v] += mb[v];
+            for (int b = 0; b < kBatch; ++b) {
+                if (k0 + b >= count) continue;
+                const int64_t slot = slot0 + 32 * static_cast<int64_t>(k0 + b);
+                load_bar<V>(face_bar + B * (2 * static_cast<int64_t>(list_face(e[b])) + (e[b] >= 0 ? 0 : 1)), mb[b]);
+                const double2 o01 = geo.off01[slot];
+                r[b][0] = o01.x;
+                r[b][1] = o01.y;
+                if constexpr (D == 3) r[b][2] = geo.off2[slot];
+            }
 #pragma unroll
-                    for (int q = 0; q < D; ++q) gi_bar[D * v + q] += r[q] * mb[v];
+            for (int b = 0; b < kBatch; ++b) {
+                if (k0 + b >= count) continue;
+                const bool fallback = !(half[0] + dot<D>(gi, r[b]) > 0 && half[P] + dot<D>(gi + D * P, r[b]) > 0);  // side_value
+                if (fallback) {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) Wi_bar[v] += mb[b][v];
+                } else {
+#pragma unroll
+                    for (int v = 0; v < V; ++v) {
+                        S[v] += mb[b][v];
+#pragma unroll
+                        for (int q = 0; q < D; ++q) gi_bar[D * v + q] += r[b][q] * mb[b][v];
+                    }
                 }
             }
         }

@@ -145,7 +145,7 @@ __global__ void __launch_bounds__(256) k_tangent_prims(int n, const double* __re
 // The limited gradient's tangent per cell at the stored fit and clip pattern (k_sweep_fit's rows and clip words), one
 // block a tile.
 template <int D>
-__global__ void __launch_bounds__(kTileCells, LUNA_ADJ_MIN_BLOCKS) k_tangent_sweep(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
+__global__ void __launch_bounds__(kTileCells, adj_min_blocks<D>()) k_tangent_sweep(MeshDev<D> m, GeometryDev<D, double> geo, int tile0,
                                                                                  const double* __restrict__ dprims, const double* __restrict__ wg,
                                                                                  const double* __restrict__ fit, const int32_t* __restrict__ clip,
                                                                                  double* __restrict__ dwg) {

@@ -117,3 +117,25 @@ def test_adjoint_config_512_against_oracle(cuda):
     grad_oracle = want[:, 2] @ dq_my + want[:, 3] @ dq_e
     grad_gpu = got[:, 2] @ dq_my + got[:, 3] @ dq_e
     assert np.max(np.abs(grad_gpu - grad_oracle)) / np.max(np.abs(grad_oracle)) < 1e-7
+
+
+def test_derivatives_on_a_mesh_with_a_many_faced_cell(cuda):
+    """A cell of 600 faces (its tile goes to the derivative sweeps' second launch) among tiny faces: the adjoint against
+    the oracle's, and the tangent as its transpose."""
+    from test_gpu_parity import ring_mesh
+
+    mesh = ring_mesh()
+    q0 = rough_state(mesh.n_cells, dim=2) * mesh.volume[:, None]
+    ora = O.OracleFV(mesh)
+    ora.set_state(q0)
+    dt = ora.time_step(0.3)
+    rng = np.random.default_rng(4)
+    qbar, dq = rng.standard_normal(q0.shape), rng.standard_normal(q0.shape) * np.abs(q0)
+    want = ora.step_adjoint(dt, qbar)
+    gpu = hydro.FiniteVolume(mesh)
+    gpu.set_state(q0)
+    got = gpu.step_adjoint(dt, qbar)
+    assert np.max(np.abs(got - want)) / np.max(np.abs(want)) < 1e-11
+    Jdq = gpu.step_tangent(dt, dq)
+    lhs, rhs = float((Jdq * qbar).sum()), float((dq * got).sum())
+    assert abs(lhs - rhs) <= 1e-12 * max(abs(lhs), abs(rhs))
