@@ -417,12 +417,13 @@ template <int D, bool Moving, bool Grad, class G, int Limit, int L = 1, int KB =
 __global__ void __launch_bounds__(kTileCells * L, MINB) k_sweep_tiles(MeshDev<D> m, GeometryDev<D, G> geo, int tile0, const double* __restrict__ prims,
                                                                G* __restrict__ grad_out, double* __restrict__ w_out, double courant,
                                                                double round_off2, Counters* __restrict__ ctr, LearnedInputs learned,
-                                                               HalfRows half, double* __restrict__ wg_out) {
+                                                               HalfRows half, double* __restrict__ wg_out, bool zero_fallbacks) {
     extern __shared__ double2 staged_rows[];
     double* rows = reinterpret_cast<double*>(staged_rows);
     constexpr int V = D + 2, GS = grad_stride<D>(), R = kStagedDoubles;
     constexpr bool exact = sizeof(G) == sizeof(double);
     static_assert(L == 1 || (Limit != 2 && 32 % L == 0), "threads a cell");
+    if (zero_fallbacks && blockIdx.x == 0 && threadIdx.x == 0) ctr->fallbacks[0] = ctr->fallbacks[1] = 0;  // for the flux pass behind
     const int tile = tile0 + static_cast<int>(blockIdx.x);
     const int in_tile = static_cast<int>(threadIdx.x) / L, sub = static_cast<int>(threadIdx.x) % L;  // the cell, the entries' share
     const int64_t t = static_cast<int64_t>(tile) * kTileCells + in_tile;

@@ -163,8 +163,10 @@ __device__ __forceinline__ void load_prim_row(const double* prims, int i, double
 }
 
 // Counters a step's kernels write; read back with dt (one copy).
+constexpr unsigned long long kNoDt = 0x7fefffffffffffffull;  // DBL_MAX: the Min reducer's identity
 struct Counters {
-    unsigned long long dt_bits;       // min over the time-step terms, as the bits of a positive double
+    unsigned long long dt_bits;       // min over the time-step terms, as the bits of a positive double; set back to kNoDt
+                                      // by the update, which follows its last reader
     unsigned long long fallbacks[2];  // face sides that took the cell's state (pass 0, moving pass 1)
     unsigned long long error;         // bit 0 non-finite dt term, bit 1 non-finite state, bit 2 index out of range
 };
@@ -615,6 +617,7 @@ template <int D, bool NextPrims, bool Windowed>
 __device__ __forceinline__ void update_cell(const MeshDev<D>& m, double* __restrict__ q, int i, const double (&sum)[D + 2], double dt,
                                             double* __restrict__ prims, const GasDev& gas, Counters* __restrict__ ctr) {
     constexpr int V = D + 2;
+    if (i == 0) ctr->dt_bits = kNoDt;
     double next[V];
     bool finite = true;
 #pragma unroll

@@ -35,7 +35,7 @@ namespace {
 // and both face states and each face's flux are formed once and shared through the block (one thread a slot recomputed
 // its neighbours': five primitives, three sets of slopes, four face states and two fluxes a slot). Measured, 512 lines of
 // 1024 cells, 200 fused steps from and to host memory: 38.5 -> 16.4 ms (the kernel 136 us a step before), the same bits.
-constexpr unsigned long long kNoDt = 0x7fefffffffffffffull;  // DBL_MAX, the Min reducer's identity
+using luna::kNoDt;
 constexpr int kLineThreads = 128, kLineHalo = 2, kLineSlots = kLineThreads - 2 * kLineHalo;
 template <int Order, bool Fused>
 __global__ void __launch_bounds__(kLineThreads) k_line_step(LineDev L, const double* __restrict__ q_all, double* __restrict__ next_all,

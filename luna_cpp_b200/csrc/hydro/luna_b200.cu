@@ -153,6 +153,8 @@ struct luna_fv {
     int64_t phase_launches[5] = {0, 0, 0, 0, 0};
 
     bool prims_ready = false, swept = false, moving_pending = false;
+    bool dt_clean = false;        // the dt word holds the reduction's identity (an update ran last)
+    bool zero_in_sweep = false;   // the next sweep also zeroes the fallback counts (a flux pass follows it)
     // The static per-face step's flux pass, launched by time_step behind the sweep with the dt of the sweep's reduction
     // read on the device (no idle gap while the host reads dt); step(dt) with that dt, bit for bit, then only updates.
     bool flux_ready = false;
@@ -517,7 +519,7 @@ luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
         if (smem > 48 * 1024) LUNA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
         kernel<<<static_cast<unsigned int>(count), luna::kTileCells * L, smem, fv->stream>>>(m, geo, static_cast<int>(first), fv->prims.ptr, grad,
                                                                                             fv->w.ptr, courant, round_off2, fv->counters.ptr, learned,
-                                                                                            half, wg_out);
+                                                                                            half, wg_out, fv->zero_in_sweep && k == 0);
         LUNA_CUDA(cudaGetLastError());
     }
     return LUNA_OK;
@@ -577,8 +579,9 @@ luna_status launch_sweep(luna_fv* fv, G* grad, double courant) {
 // sweep() (finite_volume.hpp:1107-1149): the dt word is reset, then one kernel writes gradients, point velocities and dt.
 template <int D>
 luna_status run_sweep(luna_fv* fv, double courant) {
-    const unsigned long long init = 0x7fefffffffffffffull;  // DBL_MAX: the Min reducer's identity
-    LUNA_CUDA(cudaMemcpyAsync(&fv->counters.ptr->dt_bits, &init, sizeof(init), cudaMemcpyHostToDevice, fv->stream));
+    if (!fv->dt_clean)
+        LUNA_CUDA(cudaMemcpyAsync(&fv->counters.ptr->dt_bits, &luna::kNoDt, sizeof(luna::kNoDt), cudaMemcpyHostToDevice, fv->stream));
+    fv->dt_clean = false;
     const bool moving = fv->motion == LUNA_MOVING, grad = fv->order == 1;
     if (fv->precision != LUNA_FP64) {
         if (moving) return grad ? launch_sweep<D, true, true, float>(fv, fv->grad32.ptr, courant) : launch_sweep<D, true, false, float>(fv, fv->grad32.ptr, courant);
@@ -705,6 +708,7 @@ void launch_update_rows(luna_fv* fv, double dt) {
 }
 template <int D, bool NextPrims>
 void launch_update(luna_fv* fv, double dt) {
+    fv->dt_clean = true;
     const bool small = fv->n <= kFewCells;
     if (float_flux(fv))
         small ? launch_update_rows<D, NextPrims, float, true>(fv, dt) : launch_update_rows<D, NextPrims, float, false>(fv, dt);
@@ -1510,7 +1514,13 @@ LUNA_API luna_status luna_fv_get_state(luna_fv* fv, double* q, int on_device) {
 LUNA_API luna_status luna_fv_time_step(luna_fv* fv, double courant, double* dt_out) {
     if (!fv || !dt_out) return set_error(LUNA_EINVAL, "null argument");
     if (fv->moving_pending) return set_error(LUNA_ESTATE, "time_step inside a moving step (call luna_fv_step_moving_end first)");
-    LUNA_TRY(fv->dim == 3 ? prepare_sweep<3>(fv, courant) : prepare_sweep<2>(fv, courant));
+    // (the sweep's first launch zeroes; single-cell tiles alone have no first. flux_ahead's conditions, known already)
+    const bool may_fuse = fv->precision == LUNA_FP64 && fv->order == 1 && !fv->learned_inputs && fv->fused >= 0;
+    fv->zero_in_sweep = fv->motion != LUNA_MOVING && fv->update == LUNA_UPDATE_PER_FACE && !may_fuse && fv->normal_tiles > 0;
+    const bool zeroed = fv->zero_in_sweep;
+    const luna_status swept = fv->dim == 3 ? prepare_sweep<3>(fv, courant) : prepare_sweep<2>(fv, courant);
+    fv->zero_in_sweep = false;
+    LUNA_TRY(swept);
     fv->flux_ready = false;
     bool ahead = false;
     LUNA_TRY(fv->dim == 3 ? flux_ahead<3>(fv, &ahead) : flux_ahead<2>(fv, &ahead));
@@ -1518,7 +1528,7 @@ LUNA_API luna_status luna_fv_time_step(luna_fv* fv, double courant, double* dt_o
         // the counters (dt, error word) read behind the sweep; the step's flux pass queued behind that read with the
         // reduced dt read on the device, so it runs while the host takes dt
         if (!fv->counters_read) LUNA_CUDA(cudaEventCreateWithFlags(&fv->counters_read, cudaEventDisableTiming));
-        LUNA_CUDA(cudaMemsetAsync(&fv->counters.ptr->fallbacks[0], 0, 2 * sizeof(unsigned long long), fv->stream));
+        if (!zeroed) LUNA_CUDA(cudaMemsetAsync(&fv->counters.ptr->fallbacks[0], 0, 2 * sizeof(unsigned long long), fv->stream));
         LUNA_CUDA(cudaMemcpyAsync(fv->host_counters, fv->counters.ptr, sizeof(luna::Counters), cudaMemcpyDeviceToHost, fv->stream));
         LUNA_CUDA(cudaEventRecord(fv->counters_read, fv->stream));
         luna_status st;
