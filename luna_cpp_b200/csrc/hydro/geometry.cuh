@@ -934,11 +934,6 @@ __global__ void k_apply_factors(int rows, const int* __restrict__ cells, const u
     const int s = blockIdx.x * blockDim.x + threadIdx.x;
     if (s >= rows || (count && s >= static_cast<int>(*count))) return;
     const int64_t i = cells ? cells[s] : s;
-#pragma unroll
-    for (int v = 0; v < V; ++v) {
-        const double a = alpha[5 * static_cast<int64_t>(s) + v];
-        double phi;
-        if (use_net) {
     double* p = grad + S * i + kFirst;
     double row[4 * kPieces];
 #pragma unroll
@@ -947,6 +942,11 @@ __global__ void k_apply_factors(int rows, const int* __restrict__ cells, const u
         row[c] = w.x;
         row[c + 1] = w.y;
     }
+#pragma unroll
+    for (int v = 0; v < V; ++v) {
+        const double a = alpha[5 * static_cast<int64_t>(s) + v];
+        double phi;
+        if (use_net) {
             const double o = logits[16 * static_cast<int64_t>(s) + learned_slot<D>(v)];
             phi = a / (1.0 + exp(-o));
         } else {
@@ -955,13 +955,13 @@ __global__ void k_apply_factors(int rows, const int* __restrict__ cells, const u
 #pragma unroll
         for (int d = 0; d < D; ++d) row[kPad + D * v + d] *= phi;
     }
+#pragma unroll
+    for (int c = 0; c < 4 * kPieces; c += 2) *reinterpret_cast<double2*>(p + c) = make_double2(row[c], row[c + 1]);
 }
 
 // The static flux pass over the face rows (FaceFlux::operator(), finite_volume.hpp:1415-1434): one streamed row per
 // face, then the two cells' primitive and gradient rows.
 // Resident blocks per SM the flux pass's registers are cut for; measured at 128^3 FP64 (fluxes ms): unbounded (96
-#pragma unroll
-    for (int c = 0; c < 4 * kPieces; c += 2) *reinterpret_cast<double2*>(p + c) = make_double2(row[c], row[c + 1]);
 // registers, 5 blocks) 0.80-0.84, 6 blocks 0.77 (0.699 with the later rows), 7 blocks 0.767, 8 blocks 1.03 (spills).
 #ifndef LUNA_FLUX_MIN_BLOCKS
 #define LUNA_FLUX_MIN_BLOCKS 6
@@ -1093,7 +1093,10 @@ __global__ void __launch_bounds__(kTileCells, LUNA_FUSED_MIN_BLOCKS) k_tile_flux
                 for (int v = 0; v < V; ++v) sum[v] += sign * row[b][v];
             }
         }
-        update_cell<D, true, true>(m, q, i, sum, dt, prims, x.gas, ctr);
+        double before[V];
+#pragma unroll
+        for (int v = 0; v < V; ++v) before[v] = q[V * i + v];
+        update_cell<D, true, true>(q, i, before, m.vol[i], sum, dt, prims, x.gas, ctr);
     }
     block_sum_to(static_cast<unsigned long long>(count), &ctr->fallbacks[0]);
 }
