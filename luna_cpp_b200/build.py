@@ -80,7 +80,7 @@ def build_hydro(force=False, extra=()):
     mesh = os.path.join(CSRC, "mesh")
     cu = [s for s in _sources(hydro, {".cu"})]
     remesh = os.path.join(mesh, "remesh.cu")
-    remesh_deps = [remesh] + [os.path.join(mesh, h) for h in ("voronoi_cell.h", "voronoi_grid.h")]
+    remesh_deps = [remesh] + [os.path.join(mesh, h) for h in ("voronoi_cell.h", "voronoi_grid.h", "cell_lanes.cuh")]
     deps = _sources(hydro, {".cu", ".cuh", ".h", ".hpp"}) + _sources(INCLUDE, {".h"}) + remesh_deps
     if not cu:
         return None

@@ -4,7 +4,7 @@
 // the cells have the host builder's bits). The rest is assembly in the host builder's order, done with scans and
 // per-segment sorts instead of its serial passes:
 //   buckets   counts (atomics), an exclusive scan, a fill (atomics), then each bucket's items sorted by index;
-//   cells     each cell's faces, by neighbour, appended to one face buffer at an atomic cursor (a cell's faces stay
+//   cells     (3D: cell_lanes.cuh, then one thread a cell for those it leaves) each cell's faces, by neighbour, appended to one face buffer at an atomic cursor (a cell's faces stay
 //             together; where they land does not matter, every later pass addresses them through the cell);
 //   faces     per owner (the lower-numbered cell): its faces towards higher cells, numbered by a scan, and
 //   lists     per cell, every face it is a side of (f, or ~f where it is not the owner), by neighbour: a cell's records as
@@ -19,6 +19,7 @@
 
 #include "luna_b200.h"
 #include "luna_remesh.h"
+#include "cell_lanes.cuh"
 #include "voronoi_cell.h"
 #include "voronoi_grid.h"
 
@@ -84,12 +85,16 @@ struct Counters {
     int error;                        // the first cell error (voronoi_cell.h), 0: none
     int error_cell;
     int nonfinite;                    // a generator coordinate was not finite
+    unsigned int left;                // cells that the eight-lane kernels left for one thread
     unsigned int retry;               // cells the fast path handed to the far search
 };
 
 struct Box {
     double s[3];
 };
+
+constexpr bool kEightLanes = LUNA_REMESH_DUAL;  // 3D cells by cell_lanes.cuh first
+constexpr int64_t kChunk = 1 << 17;             // cells whose candidates are held at a time (277 MB)
 
 int grid_blocks(int64_t n, int per) { return static_cast<int>((n + per - 1) / per); }
 
@@ -151,7 +156,8 @@ struct CellOut {
     unsigned long long capacity;
 };
 
-// The cells (all of them, or those of the list), each built by one thread. Without Far, a cell whose search would
+// The cells (all of them, or those of the list), each built by one thread: 2D cells, and the 3D cells that cell_lanes.cuh
+// leaves (2^18 uniform random points: about half of them; a jittered lattice: none). Without Far, a cell whose search would
 // pass the grid's sorted offsets or fill the candidate store is put on the retry list for the Far pass (the same cell
 // either way, voronoi_cell.h), which keeps the common cell's code small. 1,024 threads an SM (64 registers, a few
 // spilled): 57.5 ms for the 128^3 jittered remesh against 62 ms at 80 registers, 58.6 ms at 896 threads and 58 ms at
@@ -464,7 +470,11 @@ struct luna_remesh {
     Buf<int32_t> items;
     Buf<double> volume, centroid;
     Buf<int64_t> first;
+    Buf<int32_t> left;   // cells that the eight-lane kernels left for one thread
     Buf<int32_t> retry;  // cells the fast path handed to the far search
+    Buf<double4> shell_plane;  // a chunk's candidates (Shell)
+    Buf<double> shell_d2, shell_cover;
+    Buf<int32_t> shell_j, shell_n;
     Buf<int32_t> count, fj;
     Buf<double> fa, fc;
     Buf<int32_t> fwd, flips;
@@ -560,6 +570,15 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
     RM_TRY(centroid.reserve(n * D, "centroids"));
     RM_TRY(first.reserve(n, "cell records"));
     RM_TRY(retry.reserve(n, "far cells"));
+    if constexpr (D == 3 && kEightLanes) {
+        const int64_t chunk = n < kChunk ? n : kChunk;
+        RM_TRY(left.reserve(n, "cells left"));
+        RM_TRY(shell_plane.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_d2.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_j.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_n.reserve(chunk, "candidates"));
+        RM_TRY(shell_cover.reserve(chunk, "candidates"));
+    }
     RM_TRY(count.reserve(n, "cell records"));
     RM_TRY(fwd.reserve(n, "owned faces"));
     RM_TRY(flips.reserve(n, "flipped faces"));
@@ -598,8 +617,27 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
         RM_TRY(fc.reserve(capacity * D, "face records"));
         if (attempt > 0) RM_CUDA(cudaMemsetAsync(counters.ptr, 0, sizeof(Counters), stream));
         const CellOut out{volume.ptr, centroid.ptr, first.ptr, count.ptr, fj.ptr, fa.ptr, fc.ptr, capacity};
-        k_cells<D, false><<<grid_blocks(n, 64), 64, 0, stream>>>(n, nullptr, pos.ptr, box, g, out, counters.ptr, retry.ptr);
-        RM_CUDA(cudaGetLastError());
+        int64_t one_thread = n;
+        if constexpr (D == 3 && kEightLanes) {
+            const LaneOut lanes{out.volume, out.centroid, out.first, out.count, out.fj, out.fa, out.fc, out.capacity,
+                                &counters.ptr->faces, left.ptr, &counters.ptr->left};
+            const Shell shell{shell_plane.ptr, shell_d2.ptr, shell_j.ptr, shell_n.ptr, shell_cover.ptr};
+            const double3 sides = make_double3(box.s[0], box.s[1], box.s[2]);
+            for (int64_t base = 0; base < n; base += kChunk) {
+                const int64_t cells = n - base < kChunk ? n - base : kChunk;
+                k_search<<<grid_blocks(cells, kSearchWarps), 32 * kSearchWarps, 0, stream>>>(base, cells, pos.ptr, sides, g, shell);
+                k_clip<<<grid_blocks(cells * kLanes, kClipThreads), kClipThreads, 0, stream>>>(base, cells, sides, shell, lanes);
+            }
+            RM_CUDA(cudaGetLastError());
+            RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
+            RM_CUDA(cudaStreamSynchronize(stream));
+            one_thread = h.nonfinite ? 0 : h.left;
+        }
+        if (one_thread > 0) {
+            k_cells<D, false><<<grid_blocks(one_thread, 64), 64, 0, stream>>>(one_thread, D == 3 && kEightLanes ? left.ptr : nullptr, pos.ptr, box,
+                                                                            g, out, counters.ptr, retry.ptr);
+            RM_CUDA(cudaGetLastError());
+        }
         RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
         RM_CUDA(cudaStreamSynchronize(stream));
         if (h.retry > 0 && !h.error && !h.nonfinite) {  // the far search for the cells the fast path handed on
@@ -700,7 +738,8 @@ LUNA_API luna_status luna_remesh_device_bytes(const luna_remesh* r, int64_t* out
     if (!r || !out) return fail(LUNA_EINVAL, "luna_remesh_device_bytes: null argument");
     const size_t b = r->offsets.bytes() + r->bound2.bytes() + r->input.bytes() + r->pos.bytes() + r->bucket.bytes() +
                      r->bucket_start.bytes() + r->bucket_count.bytes() + r->cursor.bytes() + r->items.bytes() + r->volume.bytes() +
-                     r->centroid.bytes() + r->first.bytes() + r->retry.bytes() + r->count.bytes() + r->fj.bytes() + r->fa.bytes() + r->fc.bytes() +
+                     r->centroid.bytes() + r->first.bytes() + r->retry.bytes() + r->left.bytes() + r->shell_plane.bytes() + r->shell_d2.bytes() +
+                     r->shell_cover.bytes() + r->shell_j.bytes() + r->shell_n.bytes() + r->count.bytes() + r->fj.bytes() + r->fa.bytes() + r->fc.bytes() +
                      r->fwd.bytes() + r->flips.bytes() + r->seg_length.bytes() + r->face_start.bytes() + r->owner.bytes() +
                      r->neighbour.bytes() + r->degree.bytes() + r->start.bytes() + r->list.bytes() + r->key.bytes() + r->area.bytes() +
                      r->fcen.bytes() + r->counters.bytes() + r->scan_temp.bytes();

@@ -61,6 +61,28 @@ def test_device_mesh_equals_host_builder(cuda, name, points, box):
     r.close()
 
 
+def lane_cases():
+    """What the eight-lane cells meet at their limits: a last block with one cell, more cells than one chunk holds
+    (2^17), images at equal distances, a blob whose balls hold more images than a search keeps and whose rim cells have
+    more planes than a lane cell, a box of unequal buckets."""
+    rng = np.random.default_rng(11)
+    yield "9^3 + 8 random", np.vstack([jittered_points((9, 9, 9), jitter=0.1, seed=2), rng.random((8, 3))]), (1.0, 1.0, 1.0)
+    yield "131081 random", rng.random((131081, 3)), (1.0, 1.0, 1.0)
+    yield "regular 12^3", jittered_points((12, 12, 12), jitter=0.0, seed=1), (1.0, 1.0, 1.0)
+    blob = rng.random((4000, 3))
+    blob[:800] = 0.35 + 0.3 * blob[:800]
+    yield "blob", blob, (1.0, 1.0, 1.0)
+    box = (1.0, 0.31, 0.47)
+    yield "random, box 1 x 0.31 x 0.47", rng.random((901, 3)) * np.array(box), box
+
+
+@pytest.mark.parametrize("name,points,box", list(lane_cases()), ids=[c[0] for c in lane_cases()])
+def test_cells_by_lanes_equal_host_builder(cuda, name, points, box):
+    r = Remesher(3, box)
+    assert_same_mesh(build_mesh(points, box=box), r.build(points).to_host())
+    r.close()
+
+
 def test_remesher_reuse_grows_and_shrinks(cuda):
     """One remesher, meshes of different sizes in turn (its buffers are kept and grown)."""
     r = Remesher(3, (1.0, 1.0, 1.0))
