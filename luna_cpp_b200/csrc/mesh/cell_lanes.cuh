@@ -22,7 +22,8 @@
 namespace luna_voronoi {
 
 constexpr int kLanes = 8;         // threads a cell in k_clip
-constexpr int kFound = 96;        // images a search holds (a lattice cell's first ball has 39); a denser ball is searched again at 0.6 of its radius squared
+constexpr int kFound = 96;        // images a search holds (a lattice cell's first ball has 39); a denser ball is searched
+                                  // again at 0.6 of its radius squared
 constexpr int kKept = 48;         // the nearest of them, kept for the clip (a lattice cell asks for 25)
 constexpr int kLanePlanes = 34;   // planes of a cell, the box's six among them (a lattice cell: 22)
 constexpr int kLaneVerts = 48;    // vertices of a cell (a lattice cell: 28)
@@ -398,8 +399,8 @@ __global__ void __launch_bounds__(kClipThreads, 10) k_clip(int64_t base, int64_t
     int at = 0;
     bool bad = false;
 #pragma unroll 1
-    for (int r = 0; r < RF; ++r) {  // each face's vertices in order, from its oldest (DualT::finish: there a cut keeps the vertices in order of
-                                     // age, so its lowest)
+    for (int r = 0; r < RF; ++r) {  // each face's vertices in order, from its oldest
+                                     // (DualT::finish: from its lowest, in an order that a cut keeps by age)
         const int f = l + kLanes * r;
         int p = 0, m = 0, t0 = 0;
         uint64_t has = 0;

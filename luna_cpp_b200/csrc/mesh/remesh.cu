@@ -1,11 +1,12 @@
 // The moving mesh's remesh on the device (include/luna_remesh.h).
 //
-// One thread clips one cell with the host builder's code (voronoi_cell.h; this file is compiled with -fmad=false, so
-// the cells have the host builder's bits). The rest is assembly in the host builder's order, done with scans and
+// The cells are clipped with the host builder's operations in its order (voronoi_cell.h; this file is compiled with
+// -fmad=false), so they have the host builder's bits. The rest is assembly in the host builder's order, done with scans and
 // per-segment sorts instead of its serial passes:
 //   buckets   counts (atomics), an exclusive scan, a fill (atomics), then each bucket's items sorted by index;
-//   cells     (3D: cell_lanes.cuh, then one thread a cell for those it leaves) each cell's faces, by neighbour, appended to one face buffer at an atomic cursor (a cell's faces stay
-//             together; where they land does not matter, every later pass addresses them through the cell);
+//   cells     (3D: cell_lanes.cuh, eight threads a cell; the cells it leaves, and 2D, one thread a cell) each cell's faces,
+//             by neighbour, appended to one face buffer at an atomic cursor (a cell's faces stay together; where they
+//             land does not matter, every later pass addresses them through the cell);
 //   faces     per owner (the lower-numbered cell): its faces towards higher cells, numbered by a scan, and
 //   lists     per cell, every face it is a side of (f, or ~f where it is not the owner), by neighbour: a cell's records as
 //             they are (k_emit_lists). Where a higher cell sees a face that the lower one misses (degenerate vertices),
