@@ -407,7 +407,7 @@ static __global__ void __launch_bounds__(kReduceParams * kReduceGroups) k_mlp_re
         sums[1] += warp_sum[0][k];
         sums[2] += warp_sum[1][k];
     }
-    if (weight_slots) scale = 1.0f / fmaxf(sums[2], 1e-30f);
+    if (weight_slots) scale = 1.0f / (sums[2] < 1e-30f ? 1e-30f : sums[2]);  // (a NaN weight stays NaN in all that it scales)
     if (p < kParams) g[p] = scale * sums[0];
     if (p == 0) *loss = scale * sums[1];
 }

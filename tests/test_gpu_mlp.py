@@ -223,3 +223,21 @@ def test_gradient_over_blocks_and_turns(cuda, n):
     assert abs(mean_loss - loss) <= 1e-6 * abs(loss) and rel(mean_g, g) < 1e-6
     net.gradient(xd, td, wd)
     assert np.array_equal(net.grad.cpu().numpy(), mean_g)
+
+
+@pytest.mark.parametrize("bad", [np.nan, np.inf])
+def test_weights_that_are_not_finite_show_in_all_of_the_mean_gradient(cuda, bad):
+    """The mean's scale is one over the sum of the weights: a NaN among them makes the loss and every entry of the gradient
+    NaN (a scale taken from it would leave the entries that the bad row does not reach finite and huge); an infinite one
+    leaves no finite entry but zeros."""
+    import torch
+
+    from luna_cpp_b200.learned import LimiterMLP, init_params
+
+    x, t, w = data(300)
+    w[100, 2] = bad
+    net = LimiterMLP(init_params(3))
+    loss = net.gradient(torch.tensor(x, device="cuda").to(torch.bfloat16), torch.tensor(t, device="cuda"), torch.tensor(w, device="cuda")).item()
+    g = net.grad.cpu().numpy()
+    assert np.isnan(loss)
+    assert np.all(np.isnan(g) | (g == 0)) if np.isinf(bad) else np.all(np.isnan(g))
