@@ -493,6 +493,18 @@ luna_status run_primitives(luna_fv* fv) {
     return LUNA_OK;
 }
 
+// Before a launch with `bytes` of dynamic shared memory past the 48 KB a kernel has by default. The limit is the kernel's
+// and not the launch's, so it is always raised to `most`, what any mesh may ask of this kernel: raised to each launch's own
+// need, one thread's solver could lower it between another's call and its launch, which then failed.
+template <class Kernel>
+luna_status allow_shared(Kernel kernel, size_t bytes, size_t most) {
+    if (bytes <= 48 * 1024) return LUNA_OK;
+    if (bytes > most) return set_error(LUNA_EINVAL, "a tile needs " + std::to_string(bytes) + " B of shared memory");
+    LUNA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(most)));
+    return LUNA_OK;
+}
+constexpr size_t kFusedShared = 200 * 1024;  // the most that the fused pass's plan takes
+
 // The sweep's launches: the tiles within the row budget, then (rare) the single-cell tiles that stage more rows.
 template <int D, bool Moving, bool Grad, class G, int Limit, int L>
 luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
@@ -516,7 +528,7 @@ luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
         const int64_t first = groups[k][0], count = groups[k][1] - groups[k][0];
         if (count <= 0) continue;
         const size_t smem = sizeof(double) * luna::kStagedDoubles * static_cast<size_t>(most_rows[k]);
-        if (smem > 48 * 1024) LUNA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)));
+        LUNA_TRY(allow_shared(kernel, smem, sizeof(double) * luna::kStagedDoubles * luna::kBigTileRows));
         kernel<<<static_cast<unsigned int>(count), luna::kTileCells * L, smem, fv->stream>>>(m, geo, static_cast<int>(first), fv->prims.ptr, grad,
                                                                                             fv->w.ptr, courant, round_off2, fv->counters.ptr, learned,
                                                                                             half, wg_out, fv->zero_in_sweep && k == 0);
@@ -737,7 +749,7 @@ luna_status plan_fused(luna_fv* fv) {
                                                    neighbour.data(), plan);
     if (!why.empty()) return LUNA_OK;
     const size_t smem = sizeof(double) * (D + 2) * static_cast<size_t>(plan.max_slots);
-    if (smem > 200 * 1024) return LUNA_OK;
+    if (smem > kFusedShared) return LUNA_OK;
     using Row = luna::FaceRow<double>;
     const size_t inner = plan.tface.size(), crossing = plan.xface.size();
     LUNA_TRY(upload(fv->fz_tstart, plan.tstart.data(), plan.tstart.size(), false, fv->stream, "fused tile starts"));
@@ -802,7 +814,7 @@ luna_status launch_fused(luna_fv* fv, const luna::FluxArgs<D, double>& x, double
         fv->close_timed(timed_);
     }
     auto kernel = luna::k_tile_flux_update<D, Riemann>;
-    if (fv->fused_smem > 48 * 1024) LUNA_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, fv->fused_smem));
+    LUNA_TRY(allow_shared(kernel, static_cast<size_t>(fv->fused_smem), kFusedShared));
     {
         const long timed_ = fv->open_timed(3);
         kernel<<<static_cast<unsigned int>(fv->tiles), luna::kTileCells, fv->fused_smem, fv->stream>>>(
@@ -1048,16 +1060,19 @@ luna_status run_adjoint(luna_fv* fv, double dt, double* qbar) {
     return LUNA_OK;
 }
 
-// launch(tiles, first tile, shared bytes) for a kernel of one block a tile that stages `row` doubles a staged cell: the
+// launch(tiles, first tile, shared bytes) for a kernel of one block a tile that stages kFitStaged doubles a staged cell: the
 // tiles within the row budget, then the others.
-template <class Launch>
-luna_status launch_tiles(luna_fv* fv, int row, const Launch& launch) {
+template <class Kernel, class Launch>
+luna_status launch_tiles(luna_fv* fv, Kernel kernel, const Launch& launch) {
+    constexpr size_t kRow = sizeof(double) * luna::kFitStaged;
     const int64_t groups[2][2] = {{0, fv->normal_tiles}, {fv->normal_tiles, fv->tiles}};
     const int most_rows[2] = {fv->normal_rows, fv->big_rows};
     for (int k = 0; k < 2; ++k) {
         const int64_t first = groups[k][0], count = groups[k][1] - groups[k][0];
         if (count <= 0) continue;
-        launch(static_cast<unsigned int>(count), static_cast<int>(first), sizeof(double) * row * static_cast<size_t>(most_rows[k]));
+        const size_t smem = kRow * static_cast<size_t>(most_rows[k]);
+        LUNA_TRY(allow_shared(kernel, smem, kRow * luna::kBigTileRows));
+        launch(static_cast<unsigned int>(count), static_cast<int>(first), smem);
         LUNA_CUDA(cudaGetLastError());
     }
     return LUNA_OK;
@@ -1076,8 +1091,7 @@ luna_status run_fit(luna_fv* fv) {
     const auto geo = fv->geometry_dev<D, double>();
     const long timed_ = fv->open_timed(1);
     auto kernel = fv->limiter == LUNA_LIMITER_NONE ? luna::k_sweep_fit<D, false> : luna::k_sweep_fit<D, true>;
-    const luna_status st = launch_tiles(fv, luna::kFitStaged, [&](unsigned int tiles, int first, size_t smem) {
-        if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+    const luna_status st = launch_tiles(fv, kernel, [&](unsigned int tiles, int first, size_t smem) {
         kernel<<<tiles, luna::kTileCells, smem, fv->stream>>>(m, geo, first, fv->prims.ptr, fv->wg64.ptr, fv->adj_fit.ptr, fv->adj_clip.ptr);
     });
     fv->close_timed(timed_);
@@ -1101,8 +1115,7 @@ luna_status run_tangent(luna_fv* fv, double dt, double* dq) {
         const long timed_ = fv->open_timed(1);
         luna::k_tangent_prims<D><<<blocks(N, 256), 256, 0, fv->stream>>>(static_cast<int>(N), fv->q.ptr, dq, fv->vol.ptr, fv->gas, fv->tan_dprims.ptr);
         auto kernel = luna::k_tangent_sweep<D>;
-        const luna_status st = launch_tiles(fv, luna::kFitStaged, [&](unsigned int tiles, int first, size_t smem) {
-            if (smem > 48 * 1024) cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
+        const luna_status st = launch_tiles(fv, kernel, [&](unsigned int tiles, int first, size_t smem) {
             kernel<<<tiles, luna::kTileCells, smem, fv->stream>>>(m, geo, first, fv->tan_dprims.ptr, fv->wg64.ptr, fv->adj_fit.ptr, fv->adj_clip.ptr,
                                                                   fv->tan_dgrad.ptr);
         });

@@ -139,3 +139,39 @@ def test_derivatives_on_a_mesh_with_a_many_faced_cell(cuda):
     Jdq = gpu.step_tangent(dt, dq)
     lhs, rhs = float((Jdq * qbar).sum()), float((dq * got).sum())
     assert abs(lhs - rhs) <= 1e-12 * max(abs(lhs), abs(rhs))
+
+
+def test_two_threads_with_tiles_of_different_size(cuda):
+    """Cells of 1,100 and of 2,200 faces: their tiles need 52 and 104 KB of shared memory in the derivatives' sweeps, 86 and
+    172 KB in the step's. Two threads, each with its own solver, run both at once, and each gets what it gets alone."""
+    import threading
+
+    from test_gpu_parity import ring_mesh
+
+    def passes(faces, count, out):
+        mesh = ring_mesh(faces)
+        rng = np.random.default_rng(faces)
+        q0 = rough_state(mesh.n_cells, dim=2) * mesh.volume[:, None]
+        bars = rng.standard_normal(q0.shape)
+        gpu = hydro.FiniteVolume(mesh)
+        try:
+            for _ in range(count):
+                gpu.set_state(q0)
+                dt = gpu.time_step(0.3)
+                got = gpu.step_adjoint(dt, bars), gpu.step_tangent(dt, bars * np.abs(q0)), gpu.get_state()
+        except hydro.LunaError as e:
+            got = e
+        out[faces] = got
+
+    alone, together = {}, {}
+    for faces in (1100, 2200):
+        passes(faces, 1, alone)
+    threads = [threading.Thread(target=passes, args=(faces, 400, together)) for faces in (1100, 2200)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    for faces in (1100, 2200):
+        assert not isinstance(together[faces], hydro.LunaError), together[faces]
+        for a, b in zip(alone[faces], together[faces]):
+            assert np.array_equal(a, b)
