@@ -259,6 +259,11 @@ LUNA_API luna_status luna_fv_device_bytes(luna_fv* fv, int64_t* out);
  * environment at the first step on a mesh: the same bits as the two-kernel pass in about 120 B a cell less device
  * memory, measured 5 % slower at 128^3 (the default is the two-kernel pass). */
 LUNA_API luna_status luna_fv_fused_pass(luna_fv* fv, int* fused, int64_t* crossing_faces);
+/* The sweep's tiles of the current mesh: who cut them (0 the host, 1 the device, 2 the device by the whole Morton key and
+ * its larger table, for meshes with cells far below the box), their number, how many of them stage more cells than the
+ * first launch's budget and so go to a second, and the most cells that one stages. The step's results do not depend on
+ * them. No counterpart in the reference. */
+LUNA_API luna_status luna_fv_tiles(luna_fv* fv, int* cut, int64_t* tiles, int64_t* second_launch, int* most_rows);
 
 /* ---- The 1D solver: hydro::FiniteVolume<1, Exec, Riemann, Precision<>> on a static line (src/hydro/finite_volume_1d.hpp).
  * A batch of `lines` independent lines sharing one geometry: n_cells generators at `positions` (any order) on [0, length],

@@ -57,6 +57,8 @@ using FaceRow = typename std::conditional<sizeof(G) == sizeof(double), FaceRow64
 // 49 -> 36 % of peak at 64^3, the 128^3 static step 1.80 -> 1.74 ms, with the compares below).
 constexpr int kStagedDoubles = 10;
 constexpr int kStagedPos = 7;
+static_assert(sizeof(double) * kStagedDoubles * kBigTileRows <= 227 * 1024, "the largest tile's rows in one block's shared memory");
+static_assert(sizeof(double) * 6 * kDeviceTileRows <= 48 * 1024, "k_geometry's staged centroids and generators, without a raised limit");
 
 template <int D, class G>
 struct GeometryDev {

@@ -120,6 +120,7 @@ struct luna_fv {
     DevArray<double> geo_angle, geo_reach2;
     int64_t tiles = 0, normal_tiles = 0;  // the sweep's tiles (tiles.h)
     int normal_rows = 0, big_rows = 0;
+    int tile_cut = 0;  // who cut them: 0 the host, 1 the device, 2 the device's wide cut
     // the learned limiter: inputs written by the sweep, the network's logits; mlp_params is the caller's device vector
     DevArray<unsigned char> lim_features;
     DevArray<double> lim_alpha;
@@ -348,6 +349,7 @@ luna_status build_geometry(luna_fv* fv, const luna::SweepTiles& tiles) {
     fv->normal_tiles = tiles.normal_tiles;
     fv->normal_rows = tiles.normal_rows;
     fv->big_rows = tiles.big_rows;
+    fv->tile_cut = 0;
     LUNA_TRY(upload(fv->geo_order, tiles.order.data(), tiles.order.size(), false, fv->stream, "sweep order"));
     LUNA_TRY(upload(fv->geo_slice_base, tiles.slice_base.data(), tiles.slice_base.size(), false, fv->stream, "slice bases"));
     LUNA_TRY(upload(fv->geo_stage_start, tiles.stage_start.data(), tiles.stage_start.size(), false, fv->stream, "tile row starts"));
@@ -372,6 +374,7 @@ luna_status build_geometry_device(luna_fv* fv, bool* done) {
     fv->normal_tiles = plan.normal_tiles;
     fv->normal_rows = plan.normal_rows;
     fv->big_rows = plan.big_rows;
+    fv->tile_cut = plan.wide ? 2 : 1;
     LUNA_TRY(fv->geo_order.alloc(static_cast<size_t>(plan.tiles) * luna::kTileCells, "sweep order"));
     LUNA_TRY(fv->geo_slice_base.alloc(static_cast<size_t>(plan.tiles) * (luna::kTileCells / 32) + 1, "slice bases"));
     LUNA_TRY(fv->geo_stage_start.alloc(static_cast<size_t>(plan.tiles) + 1, "tile row starts"));
@@ -1941,6 +1944,15 @@ LUNA_API luna_status luna_fv_fused_pass(luna_fv* fv, int* fused, int64_t* crossi
     if (!fv || !fused) return set_error(LUNA_EINVAL, "null argument");
     *fused = fv->fused == 1 ? 1 : 0;
     if (crossing_faces) *crossing_faces = fv->fused == 1 ? fv->fused_crossing : 0;
+    return LUNA_OK;
+}
+
+LUNA_API luna_status luna_fv_tiles(luna_fv* fv, int* cut, int64_t* tiles, int64_t* second_launch, int* most_rows) {
+    if (!fv || !cut) return set_error(LUNA_EINVAL, "null argument");
+    *cut = fv->tile_cut;
+    if (tiles) *tiles = fv->tiles;
+    if (second_launch) *second_launch = fv->tiles - fv->normal_tiles;
+    if (most_rows) *most_rows = fv->normal_rows > fv->big_rows ? fv->normal_rows : fv->big_rows;
     return LUNA_OK;
 }
 

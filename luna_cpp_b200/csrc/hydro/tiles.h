@@ -18,10 +18,11 @@ constexpr int kTileCells = 128;  // cells (threads) of a tile: one block
 constexpr int kTileRows = 416;   // staged rows a tile may use (33 KB of shared memory); a cell alone needing more gets a
                                  // tile of its own, swept by a second launch with more shared memory
 constexpr int kDeviceTileRows = 640;  // the same of the device cut, which takes its cells as they come and so stages
-                                      // more: 51 KB, the most that leaves four blocks an SM
+                                      // more: 51 KB, four blocks an SM as with 416 (registers hold four in 3D)
                                       // (61 x 47 x 53 cells: with 416 a tenth of the tiles were a second launch behind
                                       // the first, its 4 steps 914 us; now 839)
-constexpr int kBigTileRows = 2360;  // the most rows one block can stage (227 KB); a mesh with a larger list is refused
+constexpr int kBigTileRows = 2360;  // the most rows one block stages (184 KB of the 227 a block can have); a mesh with a
+                                    // longer list is refused
 
 struct SweepTiles {
     std::vector<int32_t> order;        // [tiles * kTileCells]: the cell of each thread, -1 for an idle one
@@ -82,7 +83,8 @@ std::string build_tile_faces(int64_t n_cells, int64_t n_faces, int64_t tiles, co
 struct DeviceTilePlan {
     int64_t tiles = 0, normal_tiles = 0, staged = 0, slots = 0;
     int normal_rows = 0, big_rows = 0;
-    bool fits = false;  // false: a tile needs more than the block can sort or stage (use the host cut)
+    bool fits = false;  // false: a tile has more neighbours than the wide cut's table, or stages too many (use the host cut)
+    bool wide = false;  // cut by the whole Morton key with the larger table
 };
 class DeviceTiler;
 DeviceTiler* device_tiler_create();

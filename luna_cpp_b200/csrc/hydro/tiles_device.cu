@@ -2,9 +2,14 @@
 //
 // One block of kTileCells threads per tile of 128 consecutive cells in Morton order. The block orders its cells by list
 // length (longest first, then Morton position), puts their lists' neighbours into a shared-memory hash table and keeps
-// each neighbour that is not a cell of the tile once: the halo, by cell index (sorted in the fill), as the host cut
-// stages it. A planning pass counts each tile's rows and its warps' longest lists; scans turn them into the row and slot
-// offsets; a filling pass repeats the table and writes the tiles.
+// each neighbour that is not a cell of the tile once: the halo, as it comes. A planning pass counts each tile's rows and
+// its warps' longest lists; scans turn them into the row and slot offsets; a filling pass repeats the table and writes the
+// tiles.
+//
+// Two cuts (struct Narrow, struct Wide): by the upper half of the Morton key with a small table, which nearly every mesh
+// takes, and by the whole key with a table of twice the size, for a mesh with cells far below its box (a cluster under a
+// thousandth of the box's side shares its upper keys, so its cells would lie in index order and a tile would reach most of
+// the cluster) or with a tile of many neighbours.
 #include <cuda_runtime.h>
 
 #include <cub/device/device_radix_sort.cuh>
@@ -66,8 +71,8 @@ struct Buf {
 struct TileCounters {
     int normal_rows;
     int big_rows;
-    int overflow;  // a tile with more list entries than kCandidates, or more rows than kBigTileRows
-    int pad;
+    int overflow;  // a tile with more list entries than kCandidates, more neighbours than the table, or more rows than kBigTileRows
+    int wide;      // the mesh is one for the wide cut: a tile past the narrow table, or kSharedKeys cells of one narrow key
 };
 
 struct Box3 {
@@ -76,12 +81,32 @@ struct Box3 {
 
 int nblocks(int64_t n, int per) { return static_cast<int>((n + per - 1) / per); }
 
-template <int D>
-__global__ void k_morton(int64_t n, const double* __restrict__ pos, Box3 box, uint32_t* __restrict__ keys, int32_t* __restrict__ cells) {
+// The narrow cut: the upper 32 bits of the Morton key (10 or 11 levels a side in 3D, 16 in 2D): half the passes of the
+// sort. A tile's distinct list neighbours are kept in a shared-memory hash table (open addressing, linear probing) of kHash
+// slots, at most kFill of them; more blocks are resident with the small one. 128^3: plan and fill 0.95 and 0.32 ms, with the
+// wide cut 1.36 and 0.55. Sides 40^3 at a ten-thousandth of the box, a whole set_mesh: 34 ms with the narrow cut alone (the
+// host cuts what it cannot), 0.55 with the wide one behind it; in the whole box 0.51.
+struct Narrow {
+    using Key = uint32_t;
+    static constexpr int kHash = 2048, kFill = 1536, kHashShift = 21;
+};
+struct Wide {
+    using Key = uint64_t;
+    static constexpr int kHash = 4096, kFill = 3072, kHashShift = 20;
+};
+template <class Cut>
+__host__ __device__ constexpr int key_bits(int dim) {
+    return sizeof(typename Cut::Key) == 4 ? 32 : dim == 3 ? 63 : 64;
+}
+// Cells that share one narrow key lie in index order: from a run of this many on, a quarter of a tile, the mesh takes the
+// wide cut.
+constexpr int kSharedKeys = 32;
+
+template <int D, class Cut>
+__global__ void k_morton(int64_t n, const double* __restrict__ pos, Box3 box, typename Cut::Key* __restrict__ keys, int32_t* __restrict__ cells) {
     const int64_t i = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
     if (i >= n) return;
-    // the top 32 of the key's bits (10 levels and more a side: a tile is 128 cells): half the passes of the sort
-    keys[i] = static_cast<uint32_t>(luna::morton_key(D, pos + D * i, box.s) >> (D == 3 ? 31 : 32));
+    keys[i] = static_cast<typename Cut::Key>(luna::morton_key(D, pos + D * i, box.s) >> (key_bits<Wide>(D) - key_bits<Cut>(D)));
     cells[i] = static_cast<int32_t>(i);
 }
 
@@ -110,22 +135,17 @@ struct FillOut {
     uint32_t* local;
 };
 
-// A tile's distinct list neighbours are kept in a shared-memory hash table (open addressing, linear probing): kHash
-// slots, at most kHashFill distinct neighbours (more send the mesh to the host cut, as a tile with too many entries does).
-constexpr int kHash = 2048;
-constexpr int kHashFill = 1536;
-__device__ __forceinline__ int hash_slot(int32_t x) { return static_cast<int>((static_cast<uint32_t>(x) * 2654435761u) >> 21); }
-
 // One tile: plan (Fill false) or fill (Fill true). Each cell's thread inserts its list's neighbours into the block's
 // table; a neighbour seen for the first time that is not a cell of the tile joins the halo, and its staged row (the tile's
 // cells first, in thread order, then the halo as it came) goes into the table beside it. The plan counts the rows; the
 // fill stages them and looks each list entry's row up. (The halo's order varies from run to run, the sweep's results do
-// not: the staged rows are copies. Sorted by cell, in a table of 4,096 slots, the two passes took 1.36 and 0.55 ms at
-// 128^3.)
-template <bool Fill>
-__global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int32_t* __restrict__ sorted_cells, MeshLists m, PlanOut plan,
-                                                            FillOut fill) {
-    constexpr int C = luna::kTileCells;
+// not: the staged rows are copies.) The plan reads the sorted keys, shifted down to the narrow ones, for runs of one key.
+template <bool Fill, class Cut>
+__global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int32_t* __restrict__ sorted_cells,
+                                                            const typename Cut::Key* __restrict__ sorted_keys, int to_narrow, MeshLists m,
+                                                            PlanOut plan, FillOut fill) {
+    constexpr int C = luna::kTileCells, kHash = Cut::kHash;
+    const auto hash_slot = [](int32_t x) { return static_cast<int>((static_cast<uint32_t>(x) * 2654435761u) >> Cut::kHashShift); };
     __shared__ int32_t key[kHash];
     __shared__ int16_t row_of[kHash];
     __shared__ int32_t halo[kHash];
@@ -138,6 +158,8 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
     const int len = c >= 0 ? m.start[c + 1] - m.start[c] : -1;
     own_cell[k] = c;
     own_len[k] = len;
+    if constexpr (!Fill)
+        if (idx + kSharedKeys < n && sorted_keys[idx] >> to_narrow == sorted_keys[idx + kSharedKeys] >> to_narrow) plan.ctr->wide = 1;
     for (int q = k; q < kHash; q += C) key[q] = -1;
     if (k == 0) n_halo = n_entries = table_full = 0;
     __syncthreads();
@@ -179,7 +201,7 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
                     const int o = own_index(x);
                     if (o < 0) {
                         const int q = atomicAdd(&n_halo, 1);
-                        if (q < kHashFill) halo[q] = x;
+                        if (q < Cut::kFill) halo[q] = x;
                         row_of[h] = static_cast<int16_t>(n_own + q);
                     } else {
                         row_of[h] = static_cast<int16_t>(own_row[o]);
@@ -194,8 +216,10 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
     }
     __syncthreads();
     const int halo_n = n_halo;
-    if (n_entries > kCandidates || halo_n > kHashFill || table_full) {
-        if (!Fill && k == 0) atomicOr(&plan.ctr->overflow, 1);
+    if constexpr (!Fill)
+        if (k == 0 && (n_entries > kCandidates || halo_n > Narrow::kFill || table_full)) plan.ctr->wide = 1;
+    if (n_entries > kCandidates || halo_n > Cut::kFill || table_full) {
+        if (!Fill && k == 0) plan.ctr->overflow = 1;
         return;
     }
     const int rows = n_own + halo_n;
@@ -206,8 +230,8 @@ __global__ void __launch_bounds__(luna::kTileCells) k_tiles(int64_t n, const int
         }
         if (k == 0) {
             plan.rows[t] = rows;
-            if (rows > luna::kBigTileRows)
-                atomicOr(&plan.ctr->overflow, 1);
+            if (C + Cut::kFill > luna::kBigTileRows && rows > luna::kBigTileRows)  // (the wide cut's)
+                plan.ctr->overflow = 1;
             else
                 atomicMax(rows > luna::kDeviceTileRows ? &plan.ctr->big_rows : &plan.ctr->normal_rows, rows);
         }
@@ -300,13 +324,14 @@ namespace luna {
 
 class DeviceTiler {
 public:
-    Buf<uint32_t> keys, keys_sorted;
+    Buf<uint64_t> keys, keys_sorted;  // (the narrow cut's 32-bit keys in the first half)
     Buf<int32_t> cells, cells_sorted, rows, slice_len, normal, big, normal_before, big_before, pos, rows_u, len_u, stage_start, slice_base;
     Buf<TileCounters> ctr;
     Buf<unsigned int> bad;
     Buf<unsigned char> temp;
     MeshLists lists{};
     int64_t n = 0, T = 0;
+    bool wide = false;  // the next mesh is cut by the wide cut first: the last one asked for it
     DeviceTilePlan plan;
 
     template <class F>
@@ -322,40 +347,27 @@ public:
 DeviceTiler* device_tiler_create() { return new DeviceTiler(); }
 void device_tiler_destroy(DeviceTiler* t) { delete t; }
 
-luna_status device_tiles_plan(DeviceTiler* d, int dim, int64_t n, const double* pos, const double* box, const int32_t* start,
-                              const int32_t* list, const int32_t* owner, const int32_t* neighbour, cudaStream_t s, DeviceTilePlan* out) {
-    const int64_t T = (n + kTileCells - 1) / kTileCells;
-    d->n = n;
-    d->T = T;
-    d->lists = MeshLists{start, list, owner, neighbour};
-    TL_TRY(d->keys.reserve(n, "Morton keys"));
-    TL_TRY(d->keys_sorted.reserve(n, "Morton keys"));
-    TL_TRY(d->cells.reserve(n, "Morton order"));
-    TL_TRY(d->cells_sorted.reserve(n, "Morton order"));
-    TL_TRY(d->rows.reserve(T, "tile rows"));
-    TL_TRY(d->slice_len.reserve(4 * T, "tile slices"));
-    TL_TRY(d->normal.reserve(T + 1, "tile flags"));
-    TL_TRY(d->big.reserve(T + 1, "tile flags"));
-    TL_TRY(d->normal_before.reserve(T + 1, "tile places"));
-    TL_TRY(d->big_before.reserve(T + 1, "tile places"));
-    TL_TRY(d->pos.reserve(T, "tile places"));
-    TL_TRY(d->rows_u.reserve(T + 1, "tile rows"));
-    TL_TRY(d->len_u.reserve(4 * T + 1, "tile slices"));
-    TL_TRY(d->stage_start.reserve(T + 1, "tile row starts"));
-    TL_TRY(d->slice_base.reserve(4 * T + 1, "slice bases"));
-    TL_TRY(d->ctr.reserve(1, "tile counters"));
+// The plan by one of the cuts; *wide: whether the mesh is one for the wide cut (both find that alike).
+template <class Cut>
+static luna_status plan_cut(DeviceTiler* d, int dim, const double* pos, const double* box, cudaStream_t s, DeviceTilePlan* out, bool* wide) {
+    using Key = typename Cut::Key;
+    const int64_t n = d->n, T = d->T;
+    const int64_t words = sizeof(Key) == 8 ? n : (n + 1) / 2;
+    TL_TRY(d->keys.reserve(words, "Morton keys"));
+    TL_TRY(d->keys_sorted.reserve(words, "Morton keys"));
+    Key *keys = reinterpret_cast<Key*>(d->keys.ptr), *sorted = reinterpret_cast<Key*>(d->keys_sorted.ptr);
     const Box3 b{{box[0], box[1], dim == 3 ? box[2] : 1.0}};
     if (dim == 3)
-        k_morton<3><<<nblocks(n, 256), 256, 0, s>>>(n, pos, b, d->keys.ptr, d->cells.ptr);
+        k_morton<3, Cut><<<nblocks(n, 256), 256, 0, s>>>(n, pos, b, keys, d->cells.ptr);
     else
-        k_morton<2><<<nblocks(n, 256), 256, 0, s>>>(n, pos, b, d->keys.ptr, d->cells.ptr);
+        k_morton<2, Cut><<<nblocks(n, 256), 256, 0, s>>>(n, pos, b, keys, d->cells.ptr);
     TL_CUDA(cudaGetLastError());
     TL_TRY(d->with_temp([&](void* tmp, size_t& bytes) {
-        return cub::DeviceRadixSort::SortPairs(tmp, bytes, d->keys.ptr, d->keys_sorted.ptr, d->cells.ptr, d->cells_sorted.ptr, n, 0, 32, s);
+        return cub::DeviceRadixSort::SortPairs(tmp, bytes, keys, sorted, d->cells.ptr, d->cells_sorted.ptr, n, 0, key_bits<Cut>(dim), s);
     }));
     TL_CUDA(cudaMemsetAsync(d->ctr.ptr, 0, sizeof(TileCounters), s));
-    k_tiles<false><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(n, d->cells_sorted.ptr, d->lists, PlanOut{d->rows.ptr, d->slice_len.ptr, d->ctr.ptr},
-                                                                       FillOut{});
+    k_tiles<false, Cut><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(n, d->cells_sorted.ptr, sorted, key_bits<Cut>(dim) - 32, d->lists,
+                                                                            PlanOut{d->rows.ptr, d->slice_len.ptr, d->ctr.ptr}, FillOut{});
     TL_CUDA(cudaGetLastError());
     k_tile_flags<<<nblocks(T + 1, 256), 256, 0, s>>>(T, d->rows.ptr, d->normal.ptr, d->big.ptr);
     TL_TRY(d->with_temp([&](void* tmp, size_t& bytes) { return cub::DeviceScan::ExclusiveSum(tmp, bytes, d->normal.ptr, d->normal_before.ptr, T + 1, s); }));
@@ -380,6 +392,37 @@ luna_status device_tiles_plan(DeviceTiler* d, int dim, int64_t n, const double* 
     p.slots = static_cast<int64_t>(slices) * 32;
     p.normal_rows = h.normal_rows;
     p.big_rows = h.big_rows;
+    p.wide = sizeof(Key) == 8;
+    *wide = h.wide != 0;
+    *out = p;
+    return LUNA_OK;
+}
+
+luna_status device_tiles_plan(DeviceTiler* d, int dim, int64_t n, const double* pos, const double* box, const int32_t* start,
+                              const int32_t* list, const int32_t* owner, const int32_t* neighbour, cudaStream_t s, DeviceTilePlan* out) {
+    const int64_t T = (n + kTileCells - 1) / kTileCells;
+    d->n = n;
+    d->T = T;
+    d->lists = MeshLists{start, list, owner, neighbour};
+    TL_TRY(d->cells.reserve(n, "Morton order"));
+    TL_TRY(d->cells_sorted.reserve(n, "Morton order"));
+    TL_TRY(d->rows.reserve(T, "tile rows"));
+    TL_TRY(d->slice_len.reserve(4 * T, "tile slices"));
+    TL_TRY(d->normal.reserve(T + 1, "tile flags"));
+    TL_TRY(d->big.reserve(T + 1, "tile flags"));
+    TL_TRY(d->normal_before.reserve(T + 1, "tile places"));
+    TL_TRY(d->big_before.reserve(T + 1, "tile places"));
+    TL_TRY(d->pos.reserve(T, "tile places"));
+    TL_TRY(d->rows_u.reserve(T + 1, "tile rows"));
+    TL_TRY(d->len_u.reserve(4 * T + 1, "tile slices"));
+    TL_TRY(d->stage_start.reserve(T + 1, "tile row starts"));
+    TL_TRY(d->slice_base.reserve(4 * T + 1, "slice bases"));
+    TL_TRY(d->ctr.reserve(1, "tile counters"));
+    DeviceTilePlan p;
+    bool wide = false;
+    TL_TRY(d->wide ? plan_cut<Wide>(d, dim, pos, box, s, &p, &wide) : plan_cut<Narrow>(d, dim, pos, box, s, &p, &wide));
+    if (wide && !d->wide) TL_TRY(plan_cut<Wide>(d, dim, pos, box, s, &p, &wide));
+    d->wide = wide;
     d->plan = p;
     *out = p;
     return LUNA_OK;
@@ -393,7 +436,10 @@ luna_status device_tiles_fill(DeviceTiler* d, int32_t* order, int32_t* slice_bas
     TL_CUDA(cudaMemcpyAsync(slice_base, d->slice_base.ptr, (4 * T + 1) * sizeof(int32_t), cudaMemcpyDeviceToDevice, s));
     TL_CUDA(cudaMemsetAsync(local, 0, (d->plan.slots > 0 ? d->plan.slots : 1) * sizeof(uint32_t), s));
     const FillOut f{d->pos.ptr, d->stage_start.ptr, d->slice_base.ptr, order, stage_cells, local};
-    k_tiles<true><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(d->n, d->cells_sorted.ptr, d->lists, PlanOut{}, f);
+    if (d->plan.wide)
+        k_tiles<true, Wide><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(d->n, d->cells_sorted.ptr, nullptr, 0, d->lists, PlanOut{}, f);
+    else
+        k_tiles<true, Narrow><<<static_cast<unsigned int>(T), kTileCells, 0, s>>>(d->n, d->cells_sorted.ptr, nullptr, 0, d->lists, PlanOut{}, f);
     TL_CUDA(cudaGetLastError());
     TL_TRY(d->bad.reserve(1, "tile check"));
     TL_CUDA(cudaMemsetAsync(d->bad.ptr, 0, sizeof(unsigned int), s));

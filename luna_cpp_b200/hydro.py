@@ -79,6 +79,7 @@ SIGNATURES = {
     "luna_last_error": ([], ctypes.c_char_p),
     "luna_fv_device_bytes": ([P, P], I),
     "luna_fv_fused_pass": ([P, P, P], I),
+    "luna_fv_tiles": ([P, P, P, P, P], I),
     "luna_fv_step_moving_tangent": ([P, D64, P, P, P, P, P, P, I], I),
     "luna_fv_step_moving_adjoint": ([P, D64, P, P, P, P, P, P, I], I),
     "luna_fv_step_moving_tangent_end": ([P, D64, P, P, P, P, P, P, I], I),
@@ -447,6 +448,14 @@ class FiniteVolume:
         fused, crossing = ctypes.c_int(), ctypes.c_int64()
         check(lib().luna_fv_fused_pass(self._h, ctypes.byref(fused), ctypes.byref(crossing)))
         return bool(fused.value), int(crossing.value)
+
+    def tiles(self) -> dict:
+        """The sweep's tiles: who cut them ("host", "device", "device, wide"), how many, how many of them go to the second
+        launch, the most cells that one stages."""
+        cut, rows = ctypes.c_int(), ctypes.c_int()
+        count, second = ctypes.c_int64(), ctypes.c_int64()
+        check(lib().luna_fv_tiles(self._h, ctypes.byref(cut), ctypes.byref(count), ctypes.byref(second), ctypes.byref(rows)))
+        return {"cut": ("host", "device", "device, wide")[cut.value], "tiles": count.value, "second": second.value, "rows": rows.value}
 
     def device_bytes(self) -> int:
         out = ctypes.c_int64()

@@ -7,6 +7,7 @@ the same mesh given in host memory (tiles cut on the host). A moving step with t
 moving step with the host remesh, bit for bit.
 """
 import ctypes
+import dataclasses
 import os
 
 import numpy as np
@@ -15,7 +16,7 @@ from conftest import jittered_mesh, voronoi_invariants
 
 from luna_cpp_b200 import hydro
 from luna_cpp_b200.mesh import build_mesh, jittered_points
-from luna_cpp_b200.problems import point_blast
+from luna_cpp_b200.problems import point_blast, rough_state
 from luna_cpp_b200.remesh import Remesher
 
 pytestmark = pytest.mark.gpu
@@ -131,6 +132,57 @@ def test_static_step_on_device_tiles_equals_host_tiles(cuda, precision):
     a.close()
     b.close()
     r.close()
+
+
+class OnDevice:
+    """A host mesh's arrays in device memory, as a caller with a mesh builder of its own on the device has them."""
+
+    def __init__(self, mesh):
+        import torch
+
+        self.dim, self.n_cells, self.n_faces, self.box = mesh.dim, mesh.n_cells, mesh.n_faces, mesh.box
+        self.desc = hydro.mesh_desc(mesh, [])
+        self.arrays = {f: torch.tensor(np.ascontiguousarray(getattr(mesh, f)), device="cuda") for f in FIELDS}
+        for f, x in self.arrays.items():
+            setattr(self.desc, f, x.data_ptr())
+        self.desc.on_device = 1
+
+
+def shrunk(mesh, side):
+    """The mesh at `side` times its size, in the middle of one cell of the Morton keys' upper half. Lists, areas, volumes and
+    centroids are the mesh's; the separations across its seam are not periodic any more, so a step on it is arithmetic and
+    not physics, the same for every tiling."""
+    corner = 0.5 + np.array([2.0 ** -11, 2.0 ** -12, 2.0 ** -12]) - 0.5 * side
+    return dataclasses.replace(mesh, positions=corner + side * mesh.positions, centroid=side * mesh.centroid,
+                               face_centroid=side * mesh.face_centroid, area=side ** 2 * mesh.area, volume=side ** 3 * mesh.volume)
+
+
+@pytest.mark.parametrize("nx", [10, 17])
+def test_device_tiles_of_cells_far_below_the_box(cuda, nx):
+    """Cells that share one upper Morton key, in random order (17^3: 128 of them in index order have more distinct
+    neighbours than the small table; 10^3: nearly all the others): the device cuts such a mesh by the whole key, the step
+    has the host tiles' bits, and a solver goes from one cut to the other with its mesh."""
+    points = jittered_points((nx,) * 3, jitter=0.1, seed=2)
+    wide = build_mesh(points[np.random.default_rng(3).permutation(len(points))])
+    tiny = shrunk(wide, 1e-4)
+    q0 = rough_state(tiny.n_cells) * tiny.volume[:, None]
+    a, b = hydro.FiniteVolume(tiny), hydro.FiniteVolume(OnDevice(tiny))
+    assert a.tiles()["cut"] == "host" and b.tiles()["cut"] == "device, wide"
+    # the cut tried first is the one that the mesh before asked for
+    for mesh, cut in ((wide, "device, wide"), (wide, "device"), (tiny, "device, wide"), (tiny, "device, wide")):
+        b.set_mesh(OnDevice(mesh))
+        assert b.tiles()["cut"] == cut
+    assert b.tiles()["second"] == 0  # the cut by the whole key keeps neighbours together
+    a.set_state(q0)
+    b.set_state(q0)
+    for _ in range(2):
+        dt = a.time_step(0.1)
+        assert b.time_step(0.1) == dt
+        a.step(dt)
+        b.step(dt)
+    assert np.all(np.isfinite(a.get_state())) and np.array_equal(a.get_state(), b.get_state())
+    a.close()
+    b.close()
 
 
 @pytest.mark.parametrize("dim", [3, 2])
