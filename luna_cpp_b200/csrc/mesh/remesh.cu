@@ -97,6 +97,19 @@ struct Box {
 constexpr bool kEightLanes = LUNA_REMESH_DUAL;  // 3D cells by cell_lanes.cuh first
 constexpr int64_t kChunk = 1 << 17;             // cells whose candidates are held at a time (277 MB)
 
+// Few cells with a thread each are given more warps: 2^s threads a cell, of which one works, while the threads stay within
+// this many (not half of what is resident). A warp of 32 hard cells walks each one's branches in turn; a warp of one walks one.
+// Measured, a build of 512, 4,096, 16,384 and 32,768 random points, of a 20^3 lattice jittered by half its spacing and of
+// 2^18 points with a gradient of density: 3.29, 3.66, 4.26, 5.39, 2.94 and 32.0 ms with all warps full, 1.38, 2.15, 4.12, 5.27,
+// 1.30 and 24.7 with this limit; 1.37, 2.09, 3.93, 5.49, 1.29 and 24.9 with about twice as many, but 7.9 for 65,536 points
+// left by the lanes (7.2 with full warps), and 10 and 13 with four and eight times.
+constexpr int64_t kSpreadThreads = 1 << 16;
+int spread_of(int64_t cells) {
+    int s = 0;
+    while (s < 5 && cells << (s + 1) <= kSpreadThreads) ++s;
+    return s;
+}
+
 int grid_blocks(int64_t n, int per) { return static_cast<int>((n + per - 1) / per); }
 
 template <int D>
@@ -157,18 +170,19 @@ struct CellOut {
     unsigned long long capacity;
 };
 
-// The cells (all of them, or those of the list), each built by one thread: 2D cells, and the 3D cells that cell_lanes.cuh
-// leaves (2^18 uniform random points: about half of them; a jittered lattice: none). Without Far, a cell whose search would
+// The cells (all of them, or those of the list), each built by one thread, 2^spread threads a cell (spread_of): 2D cells, and
+// the 3D cells that cell_lanes.cuh leaves (uniform random points: 54 to 65 % of them; a lattice jittered by
+// 0.1: none). Without Far, a cell whose search would
 // pass the grid's sorted offsets or fill the candidate store is put on the retry list for the Far pass (the same cell
 // either way, voronoi_cell.h), which keeps the common cell's code small. 1,024 threads an SM (64 registers, a few
 // spilled): 57.5 ms for the 128^3 jittered remesh against 62 ms at 80 registers, 58.6 ms at 896 threads and 58 ms at
 // 1,280; in 64-thread blocks (16 an SM) about 1 % faster than in 128-thread blocks, and no faster with the L1 carveout
 // preferred.
 template <int D, bool Far>
-__global__ void __launch_bounds__(64, 16) k_cells(int64_t n, const int32_t* __restrict__ list, const double* __restrict__ pos, Box box, Grid g,
-                                               CellOut out, Counters* c, int32_t* __restrict__ retry) {
-    const int64_t k = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x;
-    if (k >= n) return;
+__global__ void __launch_bounds__(64, 16) k_cells(int64_t n, int spread, const int32_t* __restrict__ list, const double* __restrict__ pos, Box box,
+                                               Grid g, CellOut out, Counters* c, int32_t* __restrict__ retry) {
+    const int64_t t = blockIdx.x * static_cast<int64_t>(blockDim.x) + threadIdx.x, k = t >> spread;
+    if (k >= n || (t & ((1 << spread) - 1))) return;
     const int64_t i = list ? list[k] : k;
 #if LUNA_REMESH_DUAL
     using Poly = std::conditional_t<D == 3, Dual, Poly2>;
@@ -472,6 +486,7 @@ struct luna_remesh {
     Buf<double> volume, centroid;
     Buf<int64_t> first;
     Buf<int32_t> left;   // cells that the eight-lane kernels left for one thread
+    int64_t one_thread = 0;  // cells of the last build with a thread each
     Buf<int32_t> retry;  // cells the fast path handed to the far search
     Buf<double4> shell_plane;  // a chunk's candidates (Shell)
     Buf<double> shell_d2, shell_cover;
@@ -612,40 +627,47 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
     // cells: a first guess of the face records (16 a cell in 3D, 6 in 2D on a jittered lattice), grown once if short
     if (capacity == 0) capacity = static_cast<unsigned long long>(n) * (D == 3 ? 18 : 7);
     Counters h{};
+    const auto read_counters = [&]() -> luna_status {
+        RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
+        RM_CUDA(cudaStreamSynchronize(stream));
+        return LUNA_OK;
+    };
+    const bool by_lanes = D == 3 && kEightLanes;
     for (int attempt = 0; attempt < 2; ++attempt) {
         RM_TRY(fj.reserve(capacity, "face records"));
         RM_TRY(fa.reserve(capacity * D, "face records"));
         RM_TRY(fc.reserve(capacity * D, "face records"));
         if (attempt > 0) RM_CUDA(cudaMemsetAsync(counters.ptr, 0, sizeof(Counters), stream));
         const CellOut out{volume.ptr, centroid.ptr, first.ptr, count.ptr, fj.ptr, fa.ptr, fc.ptr, capacity};
-        int64_t one_thread = n;
-        if constexpr (D == 3 && kEightLanes) {
-            const LaneOut lanes{out.volume, out.centroid, out.first, out.count, out.fj, out.fa, out.fc, out.capacity,
-                                &counters.ptr->faces, left.ptr, &counters.ptr->left};
-            const Shell shell{shell_plane.ptr, shell_d2.ptr, shell_j.ptr, shell_n.ptr, shell_cover.ptr};
-            const double3 sides = make_double3(box.s[0], box.s[1], box.s[2]);
-            for (int64_t base = 0; base < n; base += kChunk) {
-                const int64_t cells = n - base < kChunk ? n - base : kChunk;
-                k_search<<<grid_blocks(cells, kSearchWarps), 32 * kSearchWarps, 0, stream>>>(base, cells, pos.ptr, sides, g, shell);
-                k_clip<<<grid_blocks(cells * kLanes, kClipThreads), kClipThreads, 0, stream>>>(base, cells, sides, shell, lanes);
+        one_thread = n;
+        if constexpr (D == 3 && kEightLanes)
+            if (by_lanes) {
+                const LaneOut lanes{out.volume, out.centroid, out.first, out.count, out.fj, out.fa, out.fc, out.capacity,
+                                    &counters.ptr->faces, left.ptr, &counters.ptr->left};
+                const Shell shell{shell_plane.ptr, shell_d2.ptr, shell_j.ptr, shell_n.ptr, shell_cover.ptr};
+                const double3 sides = make_double3(box.s[0], box.s[1], box.s[2]);
+                for (int64_t base = 0; base < n; base += kChunk) {
+                    const int64_t cells = n - base < kChunk ? n - base : kChunk;
+                    k_search<<<grid_blocks(cells, kSearchWarps), 32 * kSearchWarps, 0, stream>>>(base, cells, pos.ptr, sides, g, shell);
+                    k_clip<<<grid_blocks(cells * kLanes, kClipThreads), kClipThreads, 0, stream>>>(base, cells, sides, shell, lanes);
+                }
+                RM_CUDA(cudaGetLastError());
+                RM_TRY(read_counters());
+                one_thread = h.nonfinite ? 0 : h.left;
             }
-            RM_CUDA(cudaGetLastError());
-            RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
-            RM_CUDA(cudaStreamSynchronize(stream));
-            one_thread = h.nonfinite ? 0 : h.left;
-        }
         if (one_thread > 0) {
-            k_cells<D, false><<<grid_blocks(one_thread, 64), 64, 0, stream>>>(one_thread, D == 3 && kEightLanes ? left.ptr : nullptr, pos.ptr, box,
-                                                                            g, out, counters.ptr, retry.ptr);
+            const int spread = D == 3 && by_lanes ? spread_of(one_thread) : 0;
+            k_cells<D, false><<<grid_blocks(one_thread << spread, 64), 64, 0, stream>>>(one_thread, spread, by_lanes ? left.ptr : nullptr, pos.ptr,
+                                                                                       box, g, out, counters.ptr, retry.ptr);
             RM_CUDA(cudaGetLastError());
+            RM_TRY(read_counters());
         }
-        RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
-        RM_CUDA(cudaStreamSynchronize(stream));
         if (h.retry > 0 && !h.error && !h.nonfinite) {  // the far search for the cells the fast path handed on
-            k_cells<D, true><<<grid_blocks(h.retry, 64), 64, 0, stream>>>(h.retry, retry.ptr, pos.ptr, box, g, out, counters.ptr, nullptr);
+            const int spread = D == 3 ? spread_of(h.retry) : 0;
+            k_cells<D, true><<<grid_blocks(static_cast<int64_t>(h.retry) << spread, 64), 64, 0, stream>>>(h.retry, spread, retry.ptr, pos.ptr, box, g,
+                                                                                                         out, counters.ptr, nullptr);
             RM_CUDA(cudaGetLastError());
-            RM_CUDA(cudaMemcpyAsync(&h, counters.ptr, sizeof(Counters), cudaMemcpyDeviceToHost, stream));
-            RM_CUDA(cudaStreamSynchronize(stream));
+            RM_TRY(read_counters());
         }
         if (h.nonfinite) return fail(LUNA_EINVAL, "luna_remesh_build: non-finite point");
         if (h.error) return fail(LUNA_EINVAL, std::string("luna_remesh_build: cell ") + std::to_string(h.error_cell) + ": " + cell_error(h.error));
@@ -732,6 +754,12 @@ LUNA_API luna_status luna_remesh_points(luna_remesh* r, int64_t n, double** poin
     if (n < 2 || n >= (int64_t(1) << 30)) return fail(LUNA_EINVAL, "luna_remesh_points: n out of range");
     RM_TRY(r->input.reserve(static_cast<size_t>(n) * r->dim, "generators"));
     *points = r->input.ptr;
+    return LUNA_OK;
+}
+
+LUNA_API luna_status luna_remesh_one_thread(const luna_remesh* r, int64_t* out) {
+    if (!r || !out) return fail(LUNA_EINVAL, "luna_remesh_one_thread: null argument");
+    *out = r->one_thread;
     return LUNA_OK;
 }
 

@@ -132,6 +132,7 @@ SIGNATURES = {
     "luna_remesh_points": ([P, I64, P], I),
     "luna_remesh_build": ([P, I64, P, I, P, P], I),
     "luna_remesh_device_bytes": ([P, P], I),
+    "luna_remesh_one_thread": ([P, P], I),
 }
 
 PHASES = ("primitives", "sweep", "fluxes", "update", "drift")

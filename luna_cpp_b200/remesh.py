@@ -106,6 +106,12 @@ class Remesher:
         hydro.check(hydro.lib().luna_remesh_build(self._h, n, ptr, on_device, ctypes.byref(desc), ctypes.byref(inconsistent)))
         return DeviceMesh(desc, inconsistent.value)
 
+    def one_thread_cells(self) -> int:
+        """The cells of the last build that one thread each built (3D: those that the eight-lane cells left)."""
+        out = ctypes.c_int64()
+        hydro.check(hydro.lib().luna_remesh_one_thread(self._h, ctypes.byref(out)))
+        return int(out.value)
+
     def device_bytes(self) -> int:
         out = ctypes.c_int64()
         hydro.check(hydro.lib().luna_remesh_device_bytes(self._h, ctypes.byref(out)))

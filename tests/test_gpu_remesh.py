@@ -84,6 +84,17 @@ def test_cells_by_lanes_equal_host_builder(cuda, name, points, box):
     r.close()
 
 
+@pytest.mark.parametrize("n", [2000, 40000])
+def test_cells_of_random_points_by_count(cuda, n):
+    """The lanes leave about half of the cells of random points to one thread each, spread over the warps where they are
+    few. The meshes are the host builder's."""
+    points = np.random.default_rng(n).random((n, 3))
+    r = Remesher(3, (1.0, 1.0, 1.0))
+    assert_same_mesh(build_mesh(points), r.build(points).to_host())
+    assert 0.2 * n < r.one_thread_cells() < 0.8 * n
+    r.close()
+
+
 def test_remesher_reuse_grows_and_shrinks(cuda):
     """One remesher, meshes of different sizes in turn (its buffers are kept and grown)."""
     r = Remesher(3, (1.0, 1.0, 1.0))
