@@ -40,8 +40,9 @@ LUNA_API luna_status luna_remesh_points(luna_remesh* r, int64_t n, double** poin
 LUNA_API luna_status luna_remesh_build(luna_remesh* r, int64_t n, const double* points, int on_device, luna_mesh_desc* mesh,
                                        int64_t* inconsistent);
 
-/* The cells of r's last build that had one thread each: all in 2D, else those of a 3D mesh that the eight-lane
- * cells leave (0 for a lattice with a little jitter, about half for random points). The mesh is the same either way. */
+/* The cells of r's last build that had one thread each: all in 2D, in a large rectangular lattice and of 64,000 to 151,552
+ * points as irregular as random ones, else those of a 3D mesh that the eight-lane cells leave (0 for a lattice with a
+ * little jitter, about half for random points). The mesh is the same either way. */
 LUNA_API luna_status luna_remesh_one_thread(const luna_remesh* r, int64_t* out);
 
 /* Device bytes r holds. */

@@ -87,6 +87,7 @@ struct Counters {
     int error_cell;
     int nonfinite;                    // a generator coordinate was not finite
     unsigned int left;                // cells that the eight-lane kernels left for one thread
+    unsigned int boxes, close;        // of the sampled generators: in a rectangular lattice; with a neighbour close by (k_sample)
     unsigned int retry;               // cells the fast path handed to the far search
 };
 
@@ -97,6 +98,17 @@ struct Box {
 constexpr bool kEightLanes = LUNA_REMESH_DUAL;  // 3D cells by cell_lanes.cuh first
 constexpr int64_t kChunk = 1 << 17;             // cells whose candidates are held at a time (277 MB)
 
+// Which meshes past kSampleFrom cells have one thread a cell from the start (k_sample), all measured as whole builds in ms by
+// one thread / by lanes:
+// - a rectangular lattice: 48^3 0.71 / 0.88, 64^3 1.24 / 1.92 (32^3 0.46 / 0.36: hence the limit). One thread builds such a cell
+//   of 6 planes and 26 candidates without touching most of its local memory, while the lanes' search and clip cost what
+//   they always cost (with a tenth of the spacing as jitter: 48^3 3.4 / 1.7, 64^3 7.0 / 3.8);
+// - points as irregular as random ones, of which the lanes leave half and more, while one thread a cell is one wave
+//   (1,024 an SM): 65,000 points 6.95 / 7.19, 100,000 8.5 / 8.9, 131,072 9.7 / 10.3; past that 160,000 13.6 / 11.8, 262,144
+//   18.5 / 16.1. What tells them is the share of generators with another within 0.4 of the mean spacing: 0.24 of random
+//   points, more where the density varies, 0.22 of a lattice jittered by 0.7 (48^3 7.0 / 6.85) and 0.11 by 0.5 (5.7 / 5.1).
+constexpr int64_t kSampleFrom = 64000, kOneWave = 148 * 1024;
+constexpr int kSamples = 256, kLatticeSamples = 240, kIrregularSamples = 42;
 // Few cells with a thread each are given more warps: 2^s threads a cell, of which one works, while the threads stay within
 // this many (not half of what is resident). A warp of 32 hard cells walks each one's branches in turn; a warp of one walks one.
 // Measured, a build of 512, 4,096, 16,384 and 32,768 random points, of a 20^3 lattice jittered by half its spacing and of
@@ -170,8 +182,68 @@ struct CellOut {
     unsigned long long capacity;
 };
 
-// The cells (all of them, or those of the list), each built by one thread, 2^spread threads a cell (spread_of): 2D cells, and
-// the 3D cells that cell_lanes.cuh leaves (uniform random points: 54 to 65 % of them; a lattice jittered by
+// Counts, of kSamples generators spread over the mesh, those whose cell is the box between their six nearest images along
+// the axes (no other image of the 5^3 buckets around them cuts the box's corners, by the clip's own tolerance), and those
+// with another generator within 0.4 of the mean spacing. A block a generator, a thread a bucket: about 10 us, with its read.
+__global__ void __launch_bounds__(128) k_sample(int64_t n, const double* __restrict__ pos, Box box, Grid g, Counters* c) {
+    __shared__ unsigned long long nearest[7];  // of the images along each axis, on its low side and its high side; of all, squared
+    constexpr unsigned long long kNone = 0x7fefffffffffffffull;
+    const int64_t i = n * blockIdx.x / gridDim.x;
+    const int o = static_cast<int>(threadIdx.x) < 125 ? static_cast<int>(threadIdx.x) : 62;  // (the last three: the middle again)
+    const int off[3] = {o / 25 - 2, o / 5 % 5 - 2, o % 5 - 2};
+    double x[3], shift[3], scale = 0, share = 1.0 / n;  // share: the volume of a generator
+    int64_t b = 0;
+    for (int a = 0; a < 3; ++a) {
+        x[a] = pos[3 * i + a];
+        share *= box.s[a];
+        scale = box.s[a] > scale ? box.s[a] : scale;
+        int t = bucket_of(g, pos + 3 * i, a) + off[a], wraps = 0;
+        for (; t < 0; t += g.nb[a]) --wraps;
+        for (; t >= g.nb[a]; t -= g.nb[a]) ++wraps;
+        shift[a] = wraps * box.s[a];
+        b = b * g.nb[a] + t;
+    }
+    const double eps = 1e-13 * scale;
+    const int64_t q0 = g.start[b], q1 = g.start[b + 1];
+    const auto image = [&](int64_t q, double* d) {
+        double d2 = 0;
+        for (int a = 0; a < 3; ++a) {
+            d[a] = pos[3 * static_cast<int64_t>(g.items[q]) + a] + shift[a] - x[a];
+            d2 += d[a] * d[a];
+        }
+        return d2;
+    };
+    if (threadIdx.x < 7) nearest[threadIdx.x] = kNone;
+    __syncthreads();
+    for (int64_t q = q0; q < q1; ++q) {
+        double d[3];
+        const double d2 = image(q, d);
+        if (!(d2 > 0)) continue;
+        atomicMin(&nearest[6], static_cast<unsigned long long>(__double_as_longlong(d2)));
+        for (int a = 0; a < 3; ++a)
+            if (fabs(d[(a + 1) % 3]) <= eps && fabs(d[(a + 2) % 3]) <= eps)
+                atomicMin(&nearest[2 * a + (d[a] > 0)], static_cast<unsigned long long>(__double_as_longlong(fabs(d[a]))));
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        const double d2 = __longlong_as_double(static_cast<long long>(nearest[6]));
+        if (d2 * sqrt(d2) < 0.4 * 0.4 * 0.4 * share) atomicAdd(&c->close, 1u);
+    }
+    bool cut = false;
+    for (int f = 0; f < 6; ++f) cut = cut || nearest[f] == kNone;
+    if (cut) return;  // (the whole block)
+    for (int64_t q = q0; q < q1; ++q) {
+        double d[3];
+        const double d2 = image(q, d);
+        double corner = 0;
+        for (int a = 0; a < 3; ++a) corner += fabs(d[a]) * __longlong_as_double(static_cast<long long>(nearest[2 * a + (d[a] > 0)]));
+        cut = cut || !(corner - d2 <= 2 * eps * sqrt(d2));
+    }
+    if (!__syncthreads_or(cut) && threadIdx.x == 0) atomicAdd(&c->boxes, 1u);
+}
+
+// The cells (all of them, or those of the list), each built by one thread, 2^spread threads a cell (spread_of): 2D cells, a
+// lattice's, and the 3D cells that cell_lanes.cuh leaves (uniform random points: 54 to 65 % of them; a lattice jittered by
 // 0.1: none). Without Far, a cell whose search would
 // pass the grid's sorted offsets or fill the candidate store is put on the retry list for the Far pass (the same cell
 // either way, voronoi_cell.h), which keeps the common cell's code small. 1,024 threads an SM (64 registers, a few
@@ -632,7 +704,13 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
         RM_CUDA(cudaStreamSynchronize(stream));
         return LUNA_OK;
     };
-    const bool by_lanes = D == 3 && kEightLanes;
+    bool by_lanes = D == 3 && kEightLanes;
+    if (by_lanes && n >= kSampleFrom) {
+        k_sample<<<kSamples, 128, 0, stream>>>(n, pos.ptr, box, g, counters.ptr);
+        RM_CUDA(cudaGetLastError());
+        RM_TRY(read_counters());
+        by_lanes = h.boxes < kLatticeSamples && (h.close < kIrregularSamples || n > kOneWave);
+    }
     for (int attempt = 0; attempt < 2; ++attempt) {
         RM_TRY(fj.reserve(capacity, "face records"));
         RM_TRY(fa.reserve(capacity * D, "face records"));

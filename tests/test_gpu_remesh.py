@@ -84,14 +84,31 @@ def test_cells_by_lanes_equal_host_builder(cuda, name, points, box):
     r.close()
 
 
-@pytest.mark.parametrize("n", [2000, 40000])
-def test_cells_of_random_points_by_count(cuda, n):
-    """The lanes leave about half of the cells of random points to one thread each, spread over the warps where they are
-    few. The meshes are the host builder's."""
+@pytest.mark.parametrize("cells,box,lattice", [((40, 40, 40), (1.0, 1.0, 1.0), True), ((39, 40, 41), (1.0, 1.0, 1.0), False),
+                                               ((48, 45, 50), (0.96, 0.9, 1.5), True)])
+def test_lattice_cells_take_one_thread(cuda, cells, box, lattice):
+    """A rectangular lattice of 64,000 cells or more is built by one thread a cell, a smaller one and one with a
+    thousandth of jitter by lanes, which finish every cell; the meshes are the host builder's."""
+    rng = np.random.default_rng(8)
+    r = Remesher(3, box)
+    h = np.array(box) / np.array(cells)
+    points = (np.stack(np.meshgrid(*[np.arange(n) for n in cells], indexing="ij"), -1).reshape(-1, 3) + 0.5) * h
+    assert_same_mesh(build_mesh(points, box=box), r.build(points).to_host())
+    assert r.one_thread_cells() == (len(points) if lattice else 0)
+    points += 1e-3 * h * rng.uniform(-1, 1, points.shape)
+    assert_same_mesh(build_mesh(points, box=box), r.build(points).to_host())
+    assert r.one_thread_cells() == 0
+    r.close()
+
+
+@pytest.mark.parametrize("n,share", [(2000, None), (40000, None), (63999, None), (64000, 1), (151552, 1), (151553, None)])
+def test_cells_of_random_points_by_count(cuda, n, share):
+    """The lanes leave about half of the cells of random points to one thread each (of 2,000 and of 40,000 points spread
+    over the warps); between 64,000 and one wave of threads all cells take one thread. The meshes are the host builder's."""
     points = np.random.default_rng(n).random((n, 3))
     r = Remesher(3, (1.0, 1.0, 1.0))
     assert_same_mesh(build_mesh(points), r.build(points).to_host())
-    assert 0.2 * n < r.one_thread_cells() < 0.8 * n
+    assert r.one_thread_cells() == n if share else 0.2 * n < r.one_thread_cells() < 0.8 * n
     r.close()
 
 
