@@ -68,9 +68,16 @@ LUNA_API int luna_mlp_set_wait_limit(int polls) {
     return previous;
 }
 
+// The training kernel's blocks for n rows: one wave of those that share an SM (148 of them), each taking further rows in turn,
+// so the slots stay few (8.7 MB at most).
+static int train_blocks(int64_t n) {
+    using namespace luna::mlp;
+    const int64_t turns = (n + kRowsPerBlock - 1) / kRowsPerBlock, wave = 148 * kTrainBlocksPerSm;
+    return static_cast<int>(turns < wave ? turns : wave);
+}
+
 LUNA_API int64_t luna_mlp_train_workspace_floats(int64_t n) {
-    const int64_t blocks = (n + luna::mlp::kRowsPerBlock - 1) / luna::mlp::kRowsPerBlock;
-    return blocks * (luna::mlp::kParams + 2);  // a gradient, a loss and a sum of weights a block
+    return n > 0 ? static_cast<int64_t>(train_blocks(n)) * (luna::mlp::kParams + 2) : 0;  // a gradient, a loss and a sum of weights a block
 }
 
 LUNA_API luna_status luna_mlp_forward(const float* params, const void* features, int64_t n, float* logits, void* stream) {
@@ -97,14 +104,12 @@ static luna_status train_step(const char* what, const float* params, const void*
     using namespace luna::mlp;
     if (!params || !features || !target || !weight || !grad || !loss || !workspace || n <= 0 || n >= (int64_t(1) << 31))
         return fail(LUNA_EINVAL, std::string(what) + ": bad argument");
-    const int64_t turns = (n + kRowsPerBlock - 1) / kRowsPerBlock;
-    if (workspace_floats < turns * (kParams + (mean ? 2 : 1))) return fail(LUNA_EINVAL, std::string(what) + ": workspace too small");
+    const int blocks = train_blocks(n);
+    if (workspace_floats < static_cast<int64_t>(blocks) * (kParams + (mean ? 2 : 1))) return fail(LUNA_EINVAL, std::string(what) + ": workspace too small");
     cudaStream_t s = static_cast<cudaStream_t>(stream);
     const int smem = static_cast<int>(sizeof(SmemTrain));
     const cudaError_t e = cudaFuncSetAttribute(k_mlp_train, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
     if (e != cudaSuccess) return fail(LUNA_ECUDA, std::string("k_mlp_train shared memory: ") + cudaGetErrorString(e));
-    // one wave of the blocks that share an SM, each taking further rows in turn: the slots stay few
-    const int blocks = static_cast<int>(turns < 148 * kTrainBlocksPerSm ? turns : 148 * kTrainBlocksPerSm);
     float* slots = workspace;
     float* loss_slots = workspace + static_cast<int64_t>(blocks) * kParams;
     float* weight_slots = mean ? loss_slots + blocks : nullptr;

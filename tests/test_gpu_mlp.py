@@ -241,3 +241,31 @@ def test_weights_that_are_not_finite_show_in_all_of_the_mean_gradient(cuda, bad)
     g = net.grad.cpu().numpy()
     assert np.isnan(loss)
     assert np.all(np.isnan(g) | (g == 0)) if np.isinf(bad) else np.all(np.isnan(g))
+
+
+@pytest.mark.parametrize("n", [1, 64, 65, 18944, 19009, 200000])
+def test_training_workspace_holds_the_slots_written(cuda, n):
+    """A workspace of exactly the floats asked for, which stay those of one wave of blocks (296) however many the rows: the
+    call leaves what lies behind it as it was and gives the gradient that it gives with room to spare; one float less is
+    refused."""
+    import torch
+
+    from luna_cpp_b200 import hydro
+    from luna_cpp_b200.learned import LimiterMLP, _ptr, _stream, init_params
+
+    x, t, w = data(n, seed=3)
+    w[0] = 1.0
+    net = LimiterMLP(init_params(4))
+    xd, td, wd = (torch.tensor(x, device="cuda").to(torch.bfloat16), torch.tensor(t, device="cuda"), torch.tensor(w, device="cuda"))
+    need = int(hydro.lib().luna_mlp_train_workspace_floats(n))
+    assert need == min(-(-n // 64), 296) * (M.PARAMS + 2)
+    room = torch.full((need + 1024,), 7.0, device="cuda")
+    results = []
+    for floats in (need, need + 1024):
+        hydro.check(hydro.lib().luna_mlp_train_step_mean(_ptr(net.params), _ptr(xd), _ptr(td), _ptr(wd), n, _ptr(net.grad), _ptr(net.loss),
+                                                         _ptr(room), floats, _stream()))
+        results.append(net.grad.cpu().numpy().copy())
+    assert np.array_equal(*results) and bool((room[need:] == 7.0).all())
+    with pytest.raises(hydro.LunaError):
+        hydro.check(hydro.lib().luna_mlp_train_step_mean(_ptr(net.params), _ptr(xd), _ptr(td), _ptr(wd), n, _ptr(net.grad), _ptr(net.loss),
+                                                         _ptr(room), need - 1, _stream()))
