@@ -64,14 +64,14 @@ def test_limiter_none_and_uniform_random_mesh(cuda):
     assert relative(gpu.get_state(), ora.get_state()) < 1e-12
 
 
-def ring_mesh(faces=600):
+def ring_mesh(faces=600, side=24):
     """A cell with 600 faces (a centre point inside a ring of 600 points, in a lattice background): more neighbours
     than one tile of the sweep stages, so it takes the single-cell tiles' launch with more shared memory."""
     from luna_cpp_b200.mesh import build_mesh
 
     th = np.linspace(0, 2 * np.pi, faces, endpoint=False)
     ring = np.stack([0.5 + 0.2 * np.cos(th), 0.5 + 0.2 * np.sin(th)], 1)
-    g = (np.arange(24) + 0.5) / 24
+    g = (np.arange(side) + 0.5) / side
     background = np.stack(np.meshgrid(g, g, indexing="ij"), -1).reshape(-1, 2)
     background = background[np.hypot(background[:, 0] - 0.5, background[:, 1] - 0.5) > 0.3]
     return build_mesh(np.concatenate([[[0.5, 0.5]], ring, background]), (1.0, 1.0))

@@ -73,14 +73,18 @@ def lane_cases():
     blob = rng.random((4000, 3))
     blob[:800] = 0.35 + 0.3 * blob[:800]
     yield "blob", blob, (1.0, 1.0, 1.0)
-    box = (1.0, 0.31, 0.47)
-    yield "random, box 1 x 0.31 x 0.47", rng.random((901, 3)) * np.array(box), box
+    # a peak of density: balls with more images than any of a search's five holds
+    peak = rng.random((6000, 3))
+    peak[:3000] = (0.5 + 0.05 * rng.standard_normal((3000, 3))) % 1.0
+    yield "peak", peak, (1.0, 1.0, 1.0)
 
 
 @pytest.mark.parametrize("name,points,box", list(lane_cases()), ids=[c[0] for c in lane_cases()])
 def test_cells_by_lanes_equal_host_builder(cuda, name, points, box):
     r = Remesher(3, box)
     assert_same_mesh(build_mesh(points, box=box), r.build(points).to_host())
+    left = r.one_thread_cells()  # (131,081 random points: one wave of threads, all of them)
+    assert {"9^3 + 8 random": left < 50, "131081 random": left == len(points), "regular 12^3": left == 0}.get(name, 0 < left < len(points)), left
     r.close()
 
 
@@ -209,6 +213,59 @@ def test_device_tiles_of_cells_far_below_the_box(cuda, nx):
         a.step(dt)
         b.step(dt)
     assert np.all(np.isfinite(a.get_state())) and np.array_equal(a.get_state(), b.get_state())
+    a.close()
+    b.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "single", "grad16"])
+@pytest.mark.parametrize("cells", [(31, 29, 27), (153, 131)])
+def test_device_tiles_with_one_thread_a_cell(cuda, cells, precision):
+    """Past the sizes that take several threads a cell (18,944): three steps on the device's tiles have the bits of the host's."""
+    box = tuple(c / cells[0] for c in cells)
+    r = Remesher(len(cells), box)
+    dmesh = r.build(jittered_points(cells, side=box, jitter=0.3, seed=4))
+    mesh = dmesh.to_host()
+    q0 = rough_state(mesh.n_cells, dim=mesh.dim) * mesh.volume[:, None]
+    a, b = hydro.FiniteVolume(mesh, precision=precision), hydro.FiniteVolume(dmesh, precision=precision)
+    assert a.tiles()["cut"] == "host" and b.tiles()["cut"] == "device"
+    a.set_state(q0)
+    b.set_state(q0)
+    for _ in range(3):
+        dt = a.time_step(0.3)
+        assert b.time_step(0.3) == dt
+        a.step(dt)
+        b.step(dt)
+    assert np.array_equal(a.get_state(), b.get_state())
+    for x in (a, b, r):
+        x.close()
+
+
+@pytest.mark.parametrize("precision", ["fp64", "grad32"])
+@pytest.mark.parametrize("faces,side", [(700, 24), (1400, 24), (700, 160)])
+def test_device_tiles_past_the_first_launch(cuda, faces, side, precision):
+    """A cell of many faces on a device mesh: its tile stages more than the 640 cells of the first launch (and, with 1,400
+    faces, more than 48 KB of them in the derivatives' sweeps too) and goes to the second one, with the geometry read
+    through the faces. Steps, adjoint and tangent have the bits of the host's tiles, with several threads a cell and (160^2
+    cells around it) with one."""
+    from test_gpu_parity import ring_mesh
+
+    mesh = ring_mesh(faces, side)
+    assert (mesh.n_cells > 18944) == (side == 160)
+    q0 = rough_state(mesh.n_cells, dim=2) * mesh.volume[:, None]
+    a, b = hydro.FiniteVolume(mesh, precision=precision), hydro.FiniteVolume(OnDevice(mesh), precision=precision)
+    assert b.tiles()["cut"] == "device" and b.tiles()["second"] > 0 and b.tiles()["rows"] > max(640, faces)
+    a.set_state(q0)
+    b.set_state(q0)
+    for _ in range(2):
+        dt = a.time_step(0.3)
+        assert b.time_step(0.3) == dt
+        a.step(dt)
+        b.step(dt)
+    assert np.array_equal(a.get_state(), b.get_state())
+    if precision == "fp64":
+        bars = np.random.default_rng(2).standard_normal(q0.shape)
+        assert np.array_equal(a.step_adjoint(dt, bars), b.step_adjoint(dt, bars))
+        assert np.array_equal(a.step_tangent(dt, bars * q0), b.step_tangent(dt, bars * q0))
     a.close()
     b.close()
 
