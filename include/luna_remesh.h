@@ -3,8 +3,8 @@
  * luna-cpp's moving step drifts the generators and updates the Voronoi mesh between its two flux passes
  * (FiniteVolume::move(), src/hydro/finite_volume.hpp:1212-1250: mesh_->update(x_), mesh_->update_cells(), refresh()).
  * voronoi-cpp does that update on the device by repairing the previous tetrahedralisation (README.md:92-94). This
- * library rebuilds the mesh from the drifted generators on the device instead, each cell clipped by one thread with the
- * host builder's code, so the arrays equal luna_mesh_create's (libluna_mesh) bit for bit, in the layout
+ * library rebuilds the mesh from the drifted generators on the device instead, each cell clipped by eight lanes or by one
+ * thread with the host builder's operations in its order, so the arrays equal luna_mesh_create's (libluna_mesh) bit for bit, in the layout
  * luna_fv_step_moving_end reads (faces by owner, then neighbour; lists by neighbour; ~f for a face the cell does not
  * own).
  */

@@ -832,42 +832,42 @@ __global__ void __launch_bounds__(kTileCells * L, MINB) k_sweep_tiles(MeshDev<D>
                 }
             }
             if (sub == 0) {
-            bool stored = false;
-            if constexpr (!exact)
-                if (half.rows) {
-                    store_half_row<D>(half, i, g);
-                    stored = true;
+                bool stored = false;
+                if constexpr (!exact)
+                    if (half.rows) {
+                        store_half_row<D>(half, i, g);
+                        stored = true;
+                    }
+                if constexpr (exact)
+                    if (wg_out) {  // the merged row of the static per-face step: W (as staged) then g
+                        constexpr int S = wg_stride<D>();
+                        double row[S];
+#pragma unroll
+                        for (int v = 0; v < V; ++v) row[v] = Wi[v];
+#pragma unroll
+                        for (int c = 0; c < V * D; ++c) row[V + c] = g[c];
+#pragma unroll
+                        for (int c = V + V * D; c < S; ++c) row[c] = 0.0;
+                        double2* dst = reinterpret_cast<double2*>(wg_out + static_cast<int64_t>(S) * i);
+#pragma unroll
+                        for (int c = 0; c < S; c += 2) dst[c / 2] = make_double2(row[c], row[c + 1]);
+                        stored = true;
+                    }
+                if (!stored) {  // the row in 16-B vector stores (pad zeroed)
+                    G row[GS];
+#pragma unroll
+                    for (int c = 0; c < GS; ++c) row[c] = c < V * D ? g[c] : G(0);
+                    using Vec16 = typename std::conditional<sizeof(G) == sizeof(double), double2, float4>::type;
+                    constexpr int per = 16 / static_cast<int>(sizeof(G));
+                    Vec16* out = reinterpret_cast<Vec16*>(grad_out + static_cast<int64_t>(GS) * i);
+#pragma unroll
+                    for (int c = 0; c < GS; c += per) {
+                        if constexpr (sizeof(G) == sizeof(double))
+                            out[c / per] = make_double2(row[c], row[c + 1]);
+                        else
+                            out[c / per] = make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
+                    }
                 }
-            if constexpr (exact)
-                if (wg_out) {  // the merged row of the static per-face step: W (as staged) then g
-                    constexpr int S = wg_stride<D>();
-                    double row[S];
-#pragma unroll
-                    for (int v = 0; v < V; ++v) row[v] = Wi[v];
-#pragma unroll
-                    for (int c = 0; c < V * D; ++c) row[V + c] = g[c];
-#pragma unroll
-                    for (int c = V + V * D; c < S; ++c) row[c] = 0.0;
-                    double2* dst = reinterpret_cast<double2*>(wg_out + static_cast<int64_t>(S) * i);
-#pragma unroll
-                    for (int c = 0; c < S; c += 2) dst[c / 2] = make_double2(row[c], row[c + 1]);
-                    stored = true;
-                }
-            if (!stored) {  // the row in 16-B vector stores (pad zeroed)
-                G row[GS];
-#pragma unroll
-                for (int c = 0; c < GS; ++c) row[c] = c < V * D ? g[c] : G(0);
-                using Vec16 = typename std::conditional<sizeof(G) == sizeof(double), double2, float4>::type;
-                constexpr int per = 16 / static_cast<int>(sizeof(G));
-                Vec16* out = reinterpret_cast<Vec16*>(grad_out + static_cast<int64_t>(GS) * i);
-#pragma unroll
-                for (int c = 0; c < GS; c += per) {
-                    if constexpr (sizeof(G) == sizeof(double))
-                        out[c / per] = make_double2(row[c], row[c + 1]);
-                    else
-                        out[c / per] = make_float4(row[c], row[c + 1], row[c + 2], row[c + 3]);
-                }
-            }
             }
         }
     }

@@ -676,8 +676,11 @@ __device__ __forceinline__ void update_cell(double* __restrict__ q, int i, const
 // (16^3, four steps: 205 -> 201 us).
 constexpr int kSmallUpdateBlock = 64;
 template <int D, bool NextPrims, bool Windowed = false, class FS = double, bool Small = false>
-__global__ void __launch_bounds__(Small ? kSmallUpdateBlock : 256, Small || !Windowed ? 1 : sizeof(FS) == sizeof(float) ? LUNA_UPDATE_MIN_BLOCKS_F : LUNA_UPDATE_MIN_BLOCKS) k_update(MeshDev<D> m, double* __restrict__ q, const FS* __restrict__ flux, double dt,
-                                                double* __restrict__ prims, GasDev gas, Counters* __restrict__ ctr) {
+__global__ void __launch_bounds__(Small ? kSmallUpdateBlock : 256, Small || !Windowed            ? 1
+                                                                   : sizeof(FS) == sizeof(float) ? LUNA_UPDATE_MIN_BLOCKS_F
+                                                                                                 : LUNA_UPDATE_MIN_BLOCKS)
+    k_update(MeshDev<D> m, double* __restrict__ q, const FS* __restrict__ flux, double dt, double* __restrict__ prims, GasDev gas,
+             Counters* __restrict__ ctr) {
     constexpr int V = D + 2;
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= m.n) return;

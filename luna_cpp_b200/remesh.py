@@ -2,8 +2,8 @@
 
 luna-cpp's ``FiniteVolume::move()`` (src/hydro/finite_volume.hpp:1212-1250) drifts the generators and has voronoi-cpp
 update the mesh between the two flux passes of a moving step. ``Remesher`` rebuilds that mesh from the drifted
-generators on the GPU, one thread per cell running the host builder's clipping code, so a ``DeviceMesh`` holds the same
-arrays, bit for bit, as ``luna_cpp_b200.mesh.build_mesh`` gives for the same points; ``FiniteVolume.step_moving_device``
+generators on the GPU, eight lanes or one thread a cell with the host builder's operations in its order, so a ``DeviceMesh``
+holds the same arrays, bit for bit, as ``luna_cpp_b200.mesh.build_mesh`` gives for the same points; ``FiniteVolume.step_moving_device``
 runs a whole moving step with the generators and the mesh kept on the device.
 """
 from __future__ import annotations
