@@ -658,15 +658,6 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
     RM_TRY(centroid.reserve(n * D, "centroids"));
     RM_TRY(first.reserve(n, "cell records"));
     RM_TRY(retry.reserve(n, "far cells"));
-    if constexpr (D == 3 && kEightLanes) {
-        const int64_t chunk = n < kChunk ? n : kChunk;
-        RM_TRY(left.reserve(n, "cells left"));
-        RM_TRY(shell_plane.reserve(chunk * kKept, "candidates"));
-        RM_TRY(shell_d2.reserve(chunk * kKept, "candidates"));
-        RM_TRY(shell_j.reserve(chunk * kKept, "candidates"));
-        RM_TRY(shell_n.reserve(chunk, "candidates"));
-        RM_TRY(shell_cover.reserve(chunk, "candidates"));
-    }
     RM_TRY(count.reserve(n, "cell records"));
     RM_TRY(fwd.reserve(n, "owned faces"));
     RM_TRY(flips.reserve(n, "flipped faces"));
@@ -710,6 +701,15 @@ luna_status luna_remesh::build(int64_t n, const double* points, bool on_device, 
         RM_CUDA(cudaGetLastError());
         RM_TRY(read_counters());
         by_lanes = h.boxes < kLatticeSamples && (h.close < kIrregularSamples || n > kOneWave);
+    }
+    if (by_lanes) {
+        const int64_t chunk = n < kChunk ? n : kChunk;
+        RM_TRY(left.reserve(n, "cells left"));
+        RM_TRY(shell_plane.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_d2.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_j.reserve(chunk * kKept, "candidates"));
+        RM_TRY(shell_n.reserve(chunk, "candidates"));
+        RM_TRY(shell_cover.reserve(chunk, "candidates"));
     }
     for (int attempt = 0; attempt < 2; ++attempt) {
         RM_TRY(fj.reserve(capacity, "face records"));
