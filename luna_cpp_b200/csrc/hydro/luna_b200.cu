@@ -543,7 +543,9 @@ luna_status launch_sweep_lanes(luna_fv* fv, G* grad, double courant) {
 // Four threads a cell while one thread a cell leaves SMs without a tile (148 tiles of 128 cells). Measured, a whole step in
 // us at one / four threads a cell, point blast and smooth wave: 16^3 74 / 59 and 68 / 57, 24^3 75 / 61 and 71 / 61, 32^3
 // 86 / 78 and 82 / 84, 40^3 107 / 107 and 105 / 127; 2D wave 128^2 48 / 43, 200^2 53 / 64. The update's batches of eight
-// rows likewise (k_update): 16^3 4 us, 40^3 -7 us.
+// rows likewise (k_update): 16^3 4 us, 40^3 -7 us. Near the line the other policies gain too (26^3: Grad16 74 / 43, order 0
+// 66 / 38, no limiter 69 / 48; 137^2: 36 / 31, 34 / 30, 34 / 31). The sums' order and the clip's form (min-factor) then differ
+// from a larger mesh's: the last bit of FP64.
 constexpr int64_t kFewCells = 148 * luna::kTileCells;
 template <int D, bool Moving, bool Grad, class G, int Limit>
 luna_status launch_sweep_tiles(luna_fv* fv, G* grad, double courant) {

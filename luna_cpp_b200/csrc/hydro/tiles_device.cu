@@ -83,9 +83,9 @@ int nblocks(int64_t n, int per) { return static_cast<int>((n + per - 1) / per); 
 
 // The narrow cut: the upper 32 bits of the Morton key (10 or 11 levels a side in 3D, 16 in 2D): half the passes of the
 // sort. A tile's distinct list neighbours are kept in a shared-memory hash table (open addressing, linear probing) of kHash
-// slots, at most kFill of them; more blocks are resident with the small one. 128^3: plan and fill 0.95 and 0.32 ms, with the
-// wide cut 1.36 and 0.55. Sides 40^3 at a ten-thousandth of the box, a whole set_mesh: 34 ms with the narrow cut alone (the
-// host cuts what it cannot), 0.55 with the wide one behind it; in the whole box 0.51.
+// slots, at most kFill of them; more blocks are resident with the small one. 128^3: plan and fill 0.32 and 0.95 ms (0.55 and
+// 1.36 with the large table and the halo sorted by cell). 40^3 cells at a ten-thousandth of the box, a whole set_mesh: 34 ms
+// with the narrow cut alone (the host cuts what it cannot), 0.55 with the wide one behind it; in the whole box 0.51.
 struct Narrow {
     using Key = uint32_t;
     static constexpr int kHash = 2048, kFill = 1536, kHashShift = 21;
