@@ -113,8 +113,8 @@ constexpr int kSamples = 256, kLatticeSamples = 240, kIrregularSamples = 42;
 // this many (not half of what is resident). A warp of 32 hard cells walks each one's branches in turn; a warp of one walks one.
 // Measured, a build of 512, 4,096, 16,384 and 32,768 random points, of a 20^3 lattice jittered by half its spacing and of
 // 2^18 points with a gradient of density: 3.29, 3.66, 4.26, 5.39, 2.94 and 32.0 ms with all warps full, 1.38, 2.15, 4.12, 5.27,
-// 1.30 and 24.7 with this limit; 1.37, 2.09, 3.93, 5.49, 1.29 and 24.9 with about twice as many, but 7.9 for 65,536 points
-// left by the lanes (7.2 with full warps), and 10 and 13 with four and eight times.
+// 1.30 and 24.7 with this limit; 1.37, 2.09, 3.93, 5.49, 1.29 and 24.9 with about twice as many, but then
+// 7.9 for 65,536 random points by lanes (7.2 with full warps), 10 and 13 with four and eight times as many.
 constexpr int64_t kSpreadThreads = 1 << 16;
 int spread_of(int64_t cells) {
     int s = 0;
